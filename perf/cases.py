@@ -199,7 +199,7 @@ def _mixed(case, seed, pinned=False):
     if case.get("quads") or case.get("alpha_bands"):
         a = case["alpha_tex"]
         sc.draw.addTexAlpha(rng.random((a, a)) < 0.6)
-    for k, part in enumerate(_split(_f32(S.terrain(rng, n, cell, (-e, 0.0, -e), 2.0, 2.0 * cell)), bands)):
+    for k, part in enumerate(_split(_f32(S.terrain(rng, n, cell, (-e, 0.0, -e), min(2.0, 2.0 * cell))), bands)):
         alpha = k >= bands - case.get("alpha_bands", 0)
         sc.add(part, ground, dict({f: 1 for f in flags.split()}, alpha=0) if alpha else flags, chain)
     for part in _split(_f32(S.icospheres(rng, case["spheres"], 0.2, 1.0, -sp, sp)), 2):
