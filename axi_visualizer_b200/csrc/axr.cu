@@ -2243,7 +2243,7 @@ __global__ void __launch_bounds__(256) k_shadow_setup_noalloc(GroupDev G, Shadow
 template <bool ALPHA>
 __global__ void __launch_bounds__(128, ALPHA ? 6 : 8) k_shadow_raster_noalloc(GroupDev G, ShadowParams S) {
   __shared__ GroupDev sg[1];
-  __shared__ ShadowQ<ALPHA> qs[4];
+  __shared__ SpanQ<ALPHA> qs[4];
   if (threadIdx.x == 0) sg[0] = G;
   __syncthreads();
   int w = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -88,10 +88,8 @@ __device__ __forceinline__ bool grid_sync(uint32_t *bar, uint32_t nblocks, long 
 }
 
 union WarpQueue {
-  VisQ<false> vo;
-  VisQ<true> va;
-  ShadowQ<false> so;
-  ShadowQ<true> sa;
+  SpanQ<false> o;
+  SpanQ<true> a;
 };
 
 // ---- the phases, shared by the persistent kernel and the phased graph
@@ -153,19 +151,19 @@ __device__ __forceinline__ void batch_setup(const BatchParams &B, const GroupDev
 // maps' casters, then the small triangles of the shaded views
 template <bool ALPHA>
 __device__ __forceinline__ void batch_raster(const BatchParams &B, const GroupDev *sgd, const GroupDev *sgs,
-                                             ShadowQ<ALPHA> &sq, VisQ<ALPHA> &vq, int lane) {
+                                             SpanQ<ALPHA> &q, int lane) {
   if (!ALPHA)
     for (int v = 0; v < B.nviews; v++)
       if (B.views[v].kind == VIEW_SHADED) coarse_loop(B.views[v].dp, sgd + B.views[v].goff, lane);
   for (int v = 0; v < B.nviews; v++) {
     const BatchView &V = B.views[v];
     if (V.kind == VIEW_DEPTH)
-      shadow_warp_loop<ALPHA>(V.sp, sgs + V.goff, sq, lane, ALPHA ? CTR_SH_LIST_A : CTR_SH_LIST,
+      shadow_warp_loop<ALPHA>(V.sp, sgs + V.goff, q, lane, ALPHA ? CTR_SH_LIST_A : CTR_SH_LIST,
                               ALPHA ? CTR_SH_WORK_A : CTR_SH_WORK);
   }
   for (int v = 0; v < B.nviews; v++) {
     const BatchView &V = B.views[v];
-    if (V.kind == VIEW_SHADED) raster_small_loop<ALPHA>(V.dp, sgd + V.goff, vq, lane);
+    if (V.kind == VIEW_SHADED) raster_small_loop<ALPHA>(V.dp, sgd + V.goff, q, lane);
   }
 }
 
@@ -206,8 +204,8 @@ __global__ void __launch_bounds__(128, 4) k_batch(BatchParams B) {
   stamp(B.bar, 2);
 
   // phase 2: coarse units, small triangles, shadow maps (alpha-tested first)
-  batch_raster<true>(B, sgd, sgs, q.sa, q.va, lane);
-  batch_raster<false>(B, sgd, sgs, q.so, q.vo, lane);
+  batch_raster<true>(B, sgd, sgs, q.a, lane);
+  batch_raster<false>(B, sgd, sgs, q.o, lane);
   if (!grid_sync(B.bar, B.nblocks, B.spin_limit)) return;
   stamp(B.bar, 3);
 
@@ -215,9 +213,9 @@ __global__ void __launch_bounds__(128, 4) k_batch(BatchParams B) {
   for (int v = 0; v < B.nviews; v++) {
     const BatchView &V = B.views[v];
     if (V.kind != VIEW_SHADED) continue;
-    raster_tiled_loop<true>(V.dp, sgd + V.goff, q.va, lane);
-    raster_tiled_loop<false>(V.dp, sgd + V.goff, q.vo, lane);
-    fallback_loop(V.dp, sgd + V.goff, q.vo, q.va, lane, gw, nw);
+    raster_tiled_loop<true>(V.dp, sgd + V.goff, q.a, lane);
+    raster_tiled_loop<false>(V.dp, sgd + V.goff, q.o, lane);
+    fallback_loop(V.dp, sgd + V.goff, q.o, q.a, lane, gw, nw);
   }
   if (!grid_sync(B.bar, B.nblocks, B.spin_limit)) return;
   stamp(B.bar, 4);
@@ -252,16 +250,15 @@ __global__ void __launch_bounds__(256) kb_setup(BatchParams B) {
 template <bool ALPHA>
 __global__ void __launch_bounds__(128, ALPHA ? 6 : 8) kb_raster(BatchParams B) {
   __shared__ GroupDev sgd[BATCH_TABLE], sgs[BATCH_TABLE];
-  __shared__ union Q { ShadowQ<ALPHA> s; VisQ<ALPHA> v; } qs[4];
+  __shared__ SpanQ<ALPHA> qs[4];
   load_tables(B, sgd, sgs);
-  Q &q = qs[threadIdx.x >> 5];
-  batch_raster<ALPHA>(B, sgd, sgs, q.s, q.v, threadIdx.x & 31);
+  batch_raster<ALPHA>(B, sgd, sgs, qs[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
 template <bool ALPHA>
 __global__ void __launch_bounds__(128, ALPHA ? 6 : 8) kb_tiled(BatchParams B) {
   __shared__ GroupDev sgd[BATCH_TABLE], sgs[BATCH_TABLE];
-  __shared__ VisQ<ALPHA> qs[4];
+  __shared__ SpanQ<ALPHA> qs[4];
   load_tables(B, sgd, sgs);
   for (int v = 0; v < B.nviews; v++) {
     const BatchView &V = B.views[v];
@@ -271,8 +268,8 @@ __global__ void __launch_bounds__(128, ALPHA ? 6 : 8) kb_tiled(BatchParams B) {
 
 __global__ void __launch_bounds__(128) kb_fallback(BatchParams B) {
   __shared__ GroupDev sgd[BATCH_TABLE], sgs[BATCH_TABLE];
-  __shared__ VisQ<false> qo[4];
-  __shared__ VisQ<true> qa[4];
+  __shared__ SpanQ<false> qo[4];
+  __shared__ SpanQ<true> qa[4];
   load_tables(B, sgd, sgs);
   int w = threadIdx.x >> 5, tid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int v = 0; v < B.nviews; v++) {

@@ -700,189 +700,211 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_setup(DrawParams P) {
 
 // ------------------------------------------------------------ span queue
 
-// One round of spans, one per lane, in structure-of-arrays form in shared
-// memory; the warp then fills their pixels cooperatively.  d = cx1 - cx2 and
-// rd = its reciprocal (or 0) are per span, so a pixel's t costs one multiply
-// and two fused multiply-adds instead of a division.
+// One round of a warp: every lane queues the spans of its item's next two
+// rows (row k of lane l in slot l + 32 k), structure of arrays in shared
+// memory, and the warp then fills their pixels cooperatively.  Two rows a
+// round, not one: numbering a round's pixels costs the same for both, and
+// the last, partly empty window of 32 pixels comes half as often.  Spans of
+// tall thin triangles (two pixels a row) cost the most per row, and gain most.
 template <bool ALPHA>
-struct VisQ {
-  float4 a[32];                  // cx2, d, 1/d (0: divide), cz1
-  float4 b[32];                  // cz2, pixel address - first pixel number, x - first pixel number, order
-  float4 c[ALPHA ? 32 : 1];      // u1, u2 (uv / z at the span's ends)
-  int g[ALPHA ? 32 : 1];
-  int r2l[32];                   // rank among the round's non-empty spans -> span
+struct SpanQ {
+  float4 a[64];                  // cx2, d = cx1 - cx2, RN(1 / d), cz1
+  float4 b[64];                  // cz2, ~order (views), address and x of pixel number 0
+  float4 c[ALPHA ? 64 : 1];      // u, v (times z) of the first end, of the second
+  int g[ALPHA ? 64 : 1];
+  int at[64];                    // rank among the round's non-empty spans -> byte offset of its a and b
 };
 
-// Pixels of a round are numbered 0..total-1 in span (lane) order.  Returns
-// the total, sets `pre` to this lane's first pixel number and fills the
-// rank -> span table of the non-empty spans.
-__device__ __forceinline__ int fill_prepare(int cnt, int lane, int *r2l, int &pre) {
-  int incl = cnt;
+// A lane's two rows of a round: pixel counts, address and x of the first pixel
+struct RowPair {
+  int cnt[2], addr[2], x[2];
+};
+
+// Interpolants (1 / depth) of an item whose vertices' z pass this stay in
+// [2^-31, 2^59] on every row: they run from vertex to vertex and drift by at
+// most 2^-24 of the largest a row.  Differences of such z are 0 or at least
+// 2^-53, so slopes and pixels can take the reciprocal path.
+__device__ __forceinline__ bool z_safe(float z1, float z2, float z3) {
+  return z1 >= 0x1p-30f && z2 >= 0x1p-30f && z3 >= 0x1p-30f && z1 <= 0x1p58f && z2 <= 0x1p58f && z3 <= 0x1p58f;
+}
+
+// Writes a span's ends to `slot`: first pixel lo, edges cx1 / cx2 with 1/depth
+// cz1 / cz2.  `safe`: cz1, cz2 lie in [2^-60, 2^60] and |cx2|, |d| below 2^59.
+// Every pixel x then takes t = span_t(x - cx2, d, RN(1/d)) -- exact when the
+// operands are also not too small: |d| >= 2^-60, and |cx2| >= 2^-36 or lo > 0
+// (x - cx2 is 0 or a multiple of ulp(cx2) >= 2^-59, or at least 1 - 2^-36).
+// d = +-0 means the span is the one pixel lo: its n / d is an infinity of
+// sign(n) xor sign(d), clamped to 1 or 0, or NaN for n = 0, clamped to 1; that
+// t is fixed as cx2 = lo - 1 (t = 1) or lo + 1 (t = 0) with d = 1.
+// Returns false for a span outside these ranges (real scenes almost never
+// have one); the lane then draws it alone with true divisions, and the slot
+// holds the true cx2 and d.
+template <bool ALPHA>
+__device__ __forceinline__ bool span_put(SpanQ<ALPHA> &q, int slot, bool safe, int lo, uint32_t key, float cx1,
+                                         float cx2, float cz1, float cz2, V2 cu1, V2 cu2, int g) {
+  const float d = cx1 - cx2, fl = (float)lo;
+  const bool point = d == 0.f;
+  const float n = fl - cx2;
+  const bool one = n == 0.f || (int)(__float_as_uint(n) ^ __float_as_uint(d)) >= 0;
+  const bool ok = safe && (point || (fabsf(d) >= 0x1p-60f && (fabsf(cx2) >= 0x1p-36f || lo > 0)));
+  const float qx = ok && point ? (one ? fl - 1.f : fl + 1.f) : cx2;
+  const float qd = ok && point ? 1.f : d;
+  q.a[slot] = make_float4(qx, qd, recip_rn(qd), cz1);
+  *reinterpret_cast<float2 *>(&q.b[slot]) = make_float2(cz2, __uint_as_float(key));
+  if (ALPHA) {
+    q.c[slot] = make_float4(cu1.x, cu1.y, cu2.x, cu2.y);
+    q.g[slot] = g;
+  }
+  return ok;
+}
+
+// The second half of a slot's b: address and x of pixel number 0.
+template <class Q>
+__device__ __forceinline__ void span_base(Q &q, int slot, int addr, int x) {
+  reinterpret_cast<int2 *>(&q.b[slot])[1] = make_int2(addr, x);
+}
+
+__device__ __forceinline__ unsigned bit_at(uint32_t k) {   // 1 << k, 0 for k >= 32
+  unsigned r;
+  asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(k));
+  return r;
+}
+
+// Numbers a round's pixels (lane by lane, a lane's first row before its
+// second), completes the slots and calls pix(offset, p) for every pixel number
+// p, lane j taking pixels j, j + 32, ...  A pixel's span is the last non-empty
+// one starting at or before it: its rank is the starts before the window
+// (carried along) plus those inside up to this lane (one OR-reduction of the
+// start bits).  STAGED: pix returns a state whose dependent load is in
+// flight, and `then(state)` consumes it after the next window's pix, so that
+// the load overlaps that window's lookup and arithmetic.
+template <bool STAGED, class Q, class F, class G>
+__device__ __forceinline__ void fill_rows(Q &q, int lane, const RowPair &r, F &&pix, G &&then) {
+  const int c0 = r.cnt[0], c1 = r.cnt[1];
+  int incl = c0 + c1;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     int v = __shfl_up_sync(FULL, incl, o);
     if (lane >= o) incl += v;
   }
-  pre = incl - cnt;
-  unsigned ne = __ballot_sync(FULL, cnt > 0);
-  if (cnt > 0) r2l[__popc(ne & ((1u << lane) - 1u))] = lane;
-  return __shfl_sync(FULL, incl, 31);
-}
-
-// Calls pix(span, p) for every pixel p < total, lane j taking pixels j,
-// j + 32, ...  A pixel's span is the last non-empty span starting at or
-// before it: its rank = (non-empty spans starting before the window, one
-// ballot) + (starts inside the window up to this lane, from one OR-reduction
-// of the start bits) - 1.
-template <class F>
-__device__ __forceinline__ void fill_windows(int total, int cnt, int pre, int lane, const int *r2l, F &&pix) {
-  const unsigned upto = 0xffffffffu >> (31 - lane);
-  for (int base = 0; base < total; base += 32) {
-    int rel = pre - base;
-    unsigned bit = (cnt > 0 && (unsigned)rel < 32u) ? (1u << rel) : 0u;
-    unsigned starts = __reduce_or_sync(FULL, bit);
-    int before = __popc(__ballot_sync(FULL, cnt > 0 && rel < 0));
-    int p = base + lane;
-    if (p < total) pix(r2l[before + __popc(starts & upto) - 1], p);
-  }
-}
-
-// fill_windows for a pixel function in two stages: first(span, p) issues
-// the pixel's dependent load and returns a state, second(state) consumes
-// it.  Window k's second stage runs after window k + 1's first, so the
-// load's latency overlaps the next window's lookup and arithmetic.
-template <class St, class F1, class F2>
-__device__ __forceinline__ void fill_windows2(int total, int cnt, int pre, int lane, const int *r2l, F1 &&first,
-                                              F2 &&second) {
-  const unsigned upto = 0xffffffffu >> (31 - lane);
-  St cur;
-  bool have = false;
-  for (int base = 0; base < total; base += 32) {
-    int rel = pre - base;
-    unsigned bit = (cnt > 0 && (unsigned)rel < 32u) ? (1u << rel) : 0u;
-    unsigned starts = __reduce_or_sync(FULL, bit);
-    int before = __popc(__ballot_sync(FULL, cnt > 0 && rel < 0));
-    int p = base + lane;
-    St nxt;
-    bool hn = p < total;
-    if (hn) nxt = first(r2l[before + __popc(starts & upto) - 1], p);
-    if (have) second(cur);
-    cur = nxt;
-    have = hn;
-  }
-  if (have) second(cur);
-}
-
-// One round of a span queue: numbering, the record's second half written
-// with its address and x made relative to the span's first pixel number
-// (the emitter keeps `pb` in registers until the numbering is known), then
-// the pixel-parallel fill.
-template <class Q, class F>
-__device__ __forceinline__ void fill_round(Q &q, int lane, int cnt, float4 pb, F &&pix);
-template <class St, class Q, class F1, class F2>
-__device__ __forceinline__ void fill_round2(Q &q, int lane, int cnt, float4 pb, F1 &&first, F2 &&second) {
-  int pre;
-  int total = fill_prepare(cnt, lane, q.r2l, pre);
+  const int total = __shfl_sync(FULL, incl, 31);
   if (total == 0) return;
-  if (cnt) {
-    pb.y = __int_as_float(__float_as_int(pb.y) - pre);
-    pb.z = __int_as_float(__float_as_int(pb.z) - pre);
-    q.b[lane] = pb;
+  const int pre1 = incl - c1, pre0 = pre1 - c0;
+  const unsigned n0 = __ballot_sync(FULL, c0 > 0), n1 = __ballot_sync(FULL, c1 > 0), lt = (1u << lane) - 1u;
+  int rank = __popc(n0 & lt) + __popc(n1 & lt);
+  if (c0) {
+    span_base(q, lane, r.addr[0] - pre0, r.x[0] - pre0);
+    q.at[rank++] = lane * 16;
+  }
+  if (c1) {
+    span_base(q, lane + 32, r.addr[1] - pre1, r.x[1] - pre1);
+    q.at[rank] = (lane + 32) * 16;
   }
   __syncwarp();
-  fill_windows2<St>(total, cnt, pre, lane, q.r2l, first, second);
-  __syncwarp();
-}
-template <class Q, class F>
-__device__ __forceinline__ void fill_round(Q &q, int lane, int cnt, float4 pb, F &&pix) {
-  int pre;
-  int total = fill_prepare(cnt, lane, q.r2l, pre);
-  if (total == 0) return;
-  if (cnt) {
-    pb.y = __int_as_float(__float_as_int(pb.y) - pre);
-    pb.z = __int_as_float(__float_as_int(pb.z) - pre);
-    q.b[lane] = pb;
+  uint32_t s0 = c0 ? (uint32_t)pre0 : 0x80000000u, s1 = c1 ? (uint32_t)pre1 : 0x80000000u;
+  const unsigned upto = 0xffffffffu >> (31 - lane);
+  int before = -1;
+  if constexpr (STAGED) {
+    decltype(pix(0, 0)) cur;
+    bool have = false;
+    for (int p = lane; p - lane < total; p += 32, s0 -= 32, s1 -= 32) {
+      unsigned starts = __reduce_or_sync(FULL, bit_at(s0) | bit_at(s1));
+      int k = before + __popc(starts & upto);
+      before += __popc(starts);
+      decltype(pix(0, 0)) nxt;
+      const bool hn = p < total;
+      if (hn) nxt = pix(q.at[k], p);
+      if (have) then(cur);
+      cur = nxt;
+      have = hn;
+    }
+    if (have) then(cur);
+  } else {
+    for (int p = lane; p - lane < total; p += 32, s0 -= 32, s1 -= 32) {
+      unsigned starts = __reduce_or_sync(FULL, bit_at(s0) | bit_at(s1));
+      int k = before + __popc(starts & upto);
+      before += __popc(starts);
+      if (p < total) pix(q.at[k], p);
+    }
   }
-  __syncwarp();
-  fill_windows(total, cnt, pre, lane, q.r2l, pix);
   __syncwarp();
 }
 
-// Writes lane's span record: row offset cyw, first pixel lo, ends cx1 / cx2.
-// Its second half goes to `pb`, which fill_round stores; a span that must be
-// drawn by its own lane (span_queue_form: returns false) is stored whole.
+template <class T>
+__device__ __forceinline__ const T &span_at(const T *base, int off) {
+  return *reinterpret_cast<const T *>(reinterpret_cast<const char *>(base) + off);
+}
+
+// Per-fragment visibility: the depth 1 / (interpolated 1/z), the alpha test
+// (av_draw_alpha.c:80-97), then the packed depth/order atomicMin.
+// Pixel number p of the span at byte offset `off` (x = p + b.w, address =
+// p + b.z); the depth is positive and finite there, so its key is its bits
+// with the sign set (frag_key).
 template <bool ALPHA>
-__device__ __forceinline__ bool vis_put(VisQ<ALPHA> &q, int lane, int cyw, int lo, uint32_t ord, float cx1, float cx2,
-                                        float cz1, float cz2, V2 cu1, V2 cu2, int g, float4 &pb) {
-  float qx, qd, qy;
-  bool ok = span_queue_form(cx2, cx1 - cx2, lo, qx, qd, qy);
-  q.a[lane] = make_float4(qx, qd, qy, cz1);
-  pb = make_float4(cz2, __int_as_float(cyw + lo), __int_as_float(lo), __uint_as_float(ord));
-  if (!ok) q.b[lane] = pb;
+__device__ __forceinline__ void vis_pixel(const DrawParams &P, const GroupDev *sg, const SpanQ<ALPHA> &q, int off,
+                                          int p) {
+  const float4 a = span_at(q.a, off), b = span_at(q.b, off);
+  float t = span_t((float)(p + __float_as_int(b.w)) - a.x, a.y, a.z), omt = 1 - t;
+  float tz = recip_rn(omt * b.x + t * a.w);
   if (ALPHA) {
-    q.c[lane] = make_float4(cu1.x, cu1.y, cu2.x, cu2.y);
-    q.g[lane] = g;
-  }
-  return ok;
-}
-
-// Per-fragment visibility: alpha test (av_draw_alpha.c:80-97) then the
-// packed depth/order atomicMin.
-// Pixel number p of span s (x = p + b.z, address = p + b.y).  The reciprocal
-// of the interpolated 1/z is correctly rounded (__frcp_rn), i.e. 1.0f / x.
-// DIV: a span its own lane draws, with the true division.
-template <bool ALPHA, bool DIV = false>
-__device__ __forceinline__ void vis_pixel(const DrawParams &P, const GroupDev *sg, const VisQ<ALPHA> &q, int s, int p) {
-  const float4 a = q.a[s], b = q.b[s];
-  float n = (float)(p + __float_as_int(b.z)) - a.x;
-  float t = DIV ? clamp_t(n / a.y) : span_t(n, a.y, a.z);
-  float tz = __frcp_rn((1 - t) * b.x + t * a.w);
-  if (tz != tz) return;
-  if (ALPHA) {
-    const float4 c = q.c[s];
-    const GroupDev &G = sg[q.g[s]];
-    float omt = 1 - t;
+    const float4 c = span_at(q.c, off);
+    const GroupDev &G = sg[span_at(q.g, off >> 2)];
     V2 uvi{omt * c.z + t * c.x, omt * c.w + t * c.y};
     Taps tp = make_taps(uvi, tz, G.alen, 0);
     if (!(bilerp_quad(tp, G.aquad) > 0.5f)) return;
   }
-  atomicMin((unsigned long long *)&P.keys[(size_t)(p + __float_as_int(b.y))],
-            (unsigned long long)frag_key(tz, __float_as_uint(b.w)));
+  atomicMin((unsigned long long *)&P.keys[(uint32_t)(p + __float_as_int(b.z))],
+            (unsigned long long)(__float_as_uint(tz) | 0x80000000u) << 32 | __float_as_uint(b.y));
 }
 
-// vis_pixel<true> in two stages for fill_windows2: the first stage takes
-// the depth, the alpha footprint's weights and the order key, and issues
-// the load of the packed mask quad; the second tests the bilinear alpha
-// and resolves the visibility word.
+// The span in `slot`, drawn by its lane alone with true divisions.
+template <bool ALPHA>
+__device__ __noinline__ void vis_serial(uint64_t *keys, const GroupDev *sg, const SpanQ<ALPHA> &q, int slot,
+                                        int cnt, int addr, int x) {
+  const float4 a = q.a[slot], b = q.b[slot];
+  for (int j = 0; j < cnt; j++) {
+    float t = clamp_t(((float)(x + j) - a.x) / a.y);
+    float tz = 1.0f / ((1 - t) * b.x + t * a.w);
+    if (tz != tz) continue;
+    if (ALPHA) {
+      const float4 c = q.c[slot];
+      const GroupDev &G = sg[q.g[slot]];
+      float omt = 1 - t;
+      V2 uvi{omt * c.z + t * c.x, omt * c.w + t * c.y};
+      Taps tp = make_taps(uvi, tz, G.alen, 0);
+      if (!(bilerp_quad(tp, G.aquad) > 0.5f)) continue;
+    }
+    atomicMin((unsigned long long *)&keys[(size_t)(addr + j)],
+              (unsigned long long)frag_key(tz, ~__float_as_uint(b.y)));
+  }
+}
+
+// vis_pixel<true> in two stages: the first takes the depth, the alpha
+// footprint's weights and the order key, and issues the load of the packed
+// mask quad; the second tests the bilinear alpha and resolves the word.
 struct AlphaFrag {
   unsigned long long key;
   uint32_t addr;
   unsigned m;          // the packed 2 x 2 mask quad (loaded in stage one)
   float r1, r2;        // bilinear fractions
-  bool live;
 };
-__device__ __forceinline__ AlphaFrag vis_alpha_first(const DrawParams &P, const GroupDev *sg, const VisQ<true> &q,
-                                                     int s, int p) {
+__device__ __forceinline__ AlphaFrag vis_alpha_first(const DrawParams &P, const GroupDev *sg, const SpanQ<true> &q,
+                                                     int off, int p) {
   AlphaFrag f;
-  const float4 a = q.a[s], b = q.b[s];
-  float n = (float)(p + __float_as_int(b.z)) - a.x;
-  float t = span_t(n, a.y, a.z);
-  float tz = __frcp_rn((1 - t) * b.x + t * a.w);
-  f.live = tz == tz;
-  const float4 c = q.c[s];
-  const GroupDev &G = sg[q.g[s]];
-  float omt = 1 - t;
+  const float4 a = span_at(q.a, off), b = span_at(q.b, off), c = span_at(q.c, off);
+  float t = span_t((float)(p + __float_as_int(b.w)) - a.x, a.y, a.z), omt = 1 - t;
+  float tz = recip_rn(omt * b.x + t * a.w);
+  const GroupDev &G = sg[span_at(q.g, off >> 2)];
   V2 uvi{omt * c.z + t * c.x, omt * c.w + t * c.y};
   Taps tp = make_taps(uvi, tz, G.alen, 0);
-  f.m = f.live ? (unsigned)__ldg(G.aquad + tp.tex) : 0u;
+  f.m = (unsigned)__ldg(G.aquad + tp.tex);
   f.r1 = tp.texr1;
   f.r2 = tp.texr2;
-  f.key = frag_key(tz, __float_as_uint(b.w));
-  f.addr = (uint32_t)(p + __float_as_int(b.y));
+  f.key = (unsigned long long)(__float_as_uint(tz) | 0x80000000u) << 32 | __float_as_uint(b.y);
+  f.addr = (uint32_t)(p + __float_as_int(b.z));
   return f;
 }
 __device__ __forceinline__ void vis_alpha_second(const DrawParams &P, const AlphaFrag &f) {
-  if (!f.live) return;
   float i1 = 1 - f.r1, i2 = 1 - f.r2;
   float ca = i1 * i2 * (float)(f.m & 1) + f.r1 * i2 * (float)((f.m >> 1) & 1) + i1 * f.r2 * (float)((f.m >> 2) & 1) +
              f.r1 * f.r2 * (float)((f.m >> 3) & 1);
@@ -890,24 +912,17 @@ __device__ __forceinline__ void vis_alpha_second(const DrawParams &P, const Alph
   atomicMin((unsigned long long *)&P.keys[f.addr], f.key);
 }
 
-// The lane's own span record, drawn by the lane alone with the true division.
-template <bool ALPHA>
-__device__ __forceinline__ void vis_serial(const DrawParams &P, const GroupDev *sg, const VisQ<ALPHA> &q, int lane,
-                                           int cnt) {
-  for (int j = 0; j < cnt; j++) vis_pixel<ALPHA, true>(P, sg, q, lane, j);
-}
-
-// PIPE: alpha-tested fragments through the two-stage pipeline (the small
+// STAGED: alpha-tested fragments through the two-stage pipeline (the small
 // triangles' raster: 407 -> 390 us in the 1080p frame; the tiled raster,
 // whose spans are at most 16 pixels, was 3 us slower with it).
-template <bool ALPHA, bool PIPE = false>
-__device__ __forceinline__ void vis_fill(const DrawParams &P, const GroupDev *sg, VisQ<ALPHA> &q, int lane, int cnt,
-                                         float4 pb) {
-  if constexpr (ALPHA && PIPE)
-    fill_round2<AlphaFrag>(q, lane, cnt, pb, [&](int s, int p) { return vis_alpha_first(P, sg, q, s, p); },
-                           [&](const AlphaFrag &f) { vis_alpha_second(P, f); });
+template <bool ALPHA, bool STAGED = false>
+__device__ __forceinline__ void vis_fill(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int lane,
+                                         const RowPair &r) {
+  if constexpr (ALPHA && STAGED)
+    fill_rows<true>(q, lane, r, [&](int off, int p) { return vis_alpha_first(P, sg, q, off, p); },
+                    [&](const AlphaFrag &f) { vis_alpha_second(P, f); });
   else
-    fill_round(q, lane, cnt, pb, [&](int s, int p) { vis_pixel<ALPHA>(P, sg, q, s, p); });
+    fill_rows<false>(q, lane, r, [&](int off, int p) { vis_pixel<ALPHA>(P, sg, q, off, p); }, [](int) {});
 }
 
 // ------------------------------------------------------------ small triangles
@@ -915,7 +930,7 @@ __device__ __forceinline__ void vis_fill(const DrawParams &P, const GroupDev *sg
 template <bool ALPHA>
 struct SmallLane {
   int g;
-  float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);   // second half of the last span record (fill_round stores it)
+  bool safe;       // z_safe of its vertices
   uint32_t gtri;
   int x1, x2, x3, y1, y2, y3;
   float z1, z2, z3, x4, z4;
@@ -926,7 +941,7 @@ struct SmallLane {
 
   __device__ __forceinline__ void start_half0() {
     half = 0;
-    float yd = 1.0f / (float)(y2 - y1);
+    float yd = recip_rn((float)(y2 - y1));   // (y2 == y1: the half is one row, its slopes are not used)
     s1 = (float)(x2 - x1) * yd;
     s2 = (x4 - (float)x1) * yd;
     sz1 = (z2 - z1) * yd;
@@ -950,7 +965,7 @@ struct SmallLane {
   float hs1, hs2, hsz1, hsz2;
   V2 hsu1, hsu2;
   __device__ __forceinline__ void half1_slopes() {
-    float yd = 1.0f / (float)(y3 - y2);
+    float yd = recip_rn((float)(y3 - y2));
     hs1 = (float)(x3 - x2) * yd;
     hs2 = ((float)x3 - x4) * yd;
     hsz1 = (z3 - z2) * yd;
@@ -1040,9 +1055,11 @@ struct SmallLane {
 #undef SW
     x1 = ix[0]; x2 = ix[1]; x3 = ix[2]; y1 = iy[0]; y2 = iy[1]; y3 = iy[2];
     z1 = z[0]; z2 = z[1]; z3 = z[2];
-    float yd = (float)(y2 - y1) / (float)(y3 - y1);
+    float hgt = (float)(y3 - y1);
+    float yd = quot_fast((float)(y2 - y1), hgt, recip_rn(hgt));
     x4 = (float)x1 + yd * (float)(x3 - x1);
     z4 = z1 + yd * (z3 - z1);
+    safe = z_safe(z1, z2, z3);
     if (ALPHA) {
       uv4 = add2(a[0].uv, smul2(yd, sub2(a[2].uv, a[0].uv)));
       if (G.flags & F_MIP) mip_setup<false>(a, z, true, ix, iy, nullptr, nullptr, G.tex_size, G.mip_bias);
@@ -1052,18 +1069,22 @@ struct SmallLane {
     start_half0();
   }
 
-  // writes the current row's span into q[lane], advances; returns the span's
+  // writes the current row's span into `slot`, advances; returns the span's
   // pixel count and sets `live` false after the last row
-  __device__ __forceinline__ int emit(const DrawParams &P, const GroupDev *sg, VisQ<ALPHA> &q, int lane, bool &live) {
-    int lo = 0, cnt = 0;
+  __device__ __forceinline__ int emit(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int slot, int &addr,
+                                      int &x, bool &live) {
+    int cnt = 0;
     if (cy >= 0 && cy < P.view.h) {
-      if (half == 0) span_clip(f2i(cx2), cx1, P.view.w, lo, cnt);
-      else span_clip(f2i(cx1), cx2, P.view.w, lo, cnt);
-    }
-    if (cnt && !vis_put<ALPHA>(q, lane, cy * P.view.w, lo, make_order(0, gtri, half), cx1, cx2, cz1, cz2, cu1, cu2,
-                               g, pb)) {
-      vis_serial<ALPHA>(P, sg, q, lane, cnt);
-      cnt = 0;
+      // the vertices are integers, so the edges are finite on every row
+      int lo = max(f2i(half == 0 ? cx2 : cx1), 0);
+      int hi = min(__float2int_rd(half == 0 ? cx1 : cx2), P.view.w - 1);
+      cnt = hi >= lo ? hi - lo + 1 : 0;
+      x = lo;
+      addr = cy * P.view.w + lo;
+      if (cnt && !span_put<ALPHA>(q, slot, safe, lo, ~make_order(0, gtri, half), cx1, cx2, cz1, cz2, cu1, cu2, g)) {
+        vis_serial<ALPHA>(P.keys, sg, q, slot, cnt, addr, x);
+        cnt = 0;
+      }
     }
     next_row();
     live = --left > 0;
@@ -1072,7 +1093,7 @@ struct SmallLane {
 };
 
 template <bool ALPHA>
-__device__ __forceinline__ void raster_small_loop(const DrawParams &P, const GroupDev *sg, VisQ<ALPHA> &q, int lane) {
+__device__ __forceinline__ void raster_small_loop(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int lane) {
   uint32_t n = P.ctr[ALPHA ? CTR_ITEMS_A : CTR_ITEMS];
   uint32_t cap_items = P.cap_list * MAX_CHUNKS;
   const uint32_t per = ALPHA ? claim_size(n, (uint32_t)P.claim_k) : 32u;
@@ -1094,9 +1115,10 @@ __device__ __forceinline__ void raster_small_loop(const DrawParams &P, const Gro
         if (lane == 0) atomicOr(&P.ctr[CTR_LIMIT], 1u);
         break;
       }
-      int cnt = 0;
-      if (live) cnt = L.emit(P, sg, q, lane, live);
-      vis_fill<ALPHA, true>(P, sg, q, lane, cnt, L.pb);
+      RowPair r = {};
+      if (live) r.cnt[0] = L.emit(P, sg, q, lane, r.addr[0], r.x[0], live);
+      if (live) r.cnt[1] = L.emit(P, sg, q, lane + 32, r.addr[1], r.x[1], live);
+      vis_fill<ALPHA, true>(P, sg, q, lane, r);
     }
   }
 }
@@ -1104,7 +1126,7 @@ __device__ __forceinline__ void raster_small_loop(const DrawParams &P, const Gro
 template <bool ALPHA>
 __global__ void __launch_bounds__(128, ALPHA ? 6 : 8) k_raster_small(DrawParams P) {
   __shared__ GroupDev sg[64];
-  __shared__ VisQ<ALPHA> qs[4];
+  __shared__ SpanQ<ALPHA> qs[4];
   for (int i = threadIdx.x; i < P.ngroups; i += blockDim.x) sg[i] = P.groups[i];
   __syncthreads();
   raster_small_loop<ALPHA>(P, sg, qs[threadIdx.x >> 5], threadIdx.x & 31);
@@ -1246,7 +1268,6 @@ __global__ void __launch_bounds__(128) k_coarse(DrawParams P) {
 template <bool ALPHA>
 struct TileLane {
   int g;
-  float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);   // second half of the last span record (fill_round stores it)
   uint32_t gtri;
   float x1, x2, x3, y1, y2, y3, z1, z2, z3, x4, z4;
   V2 uv1, uv2, uv3, uv4;
@@ -1305,6 +1326,8 @@ struct TileLane {
     cx1 = x3 + dy * s1; cx2 = x3 + dy * s2;
     cz1 = z3 + dy * sz1; cz2 = z3 + dy * sz2;
     if (ALPHA) { cu1 = add2(uv3, smul2(dy, su1)); cu2 = add2(uv3, smul2(dy, su2)); }
+    s1 = -s1; s2 = -s2; sz1 = -sz1; sz2 = -sz2;      // upwards: a - b is a + (-b) exactly
+    if (ALPHA) { su1 = neg2(su1); su2 = neg2(su2); }
     ybound = clampf_(y2, yMin, yMax);
     live_half = (y2 < yMax) && ((float)cy >= ybound);
   }
@@ -1354,50 +1377,50 @@ struct TileLane {
     return live_half;
   }
 
-  // queues the row's span, or draws it with the lane alone (span_queue_form);
-  // returns the pixels queued
-  __device__ __forceinline__ int put(const DrawParams &P, const GroupDev *sg, VisQ<ALPHA> &q, int lane, int lo,
-                                     int cnt) {
-    if (vis_put<ALPHA>(q, lane, cy * P.view.w, lo, make_order(1, gtri, half), cx1, cx2, cz1, cz2, cu1, cu2, g, pb))
-      return cnt;
-    vis_serial<ALPHA>(P, sg, q, lane, cnt);
+  // queues the row's span, or draws it with the lane alone; returns the
+  // pixels queued.  The vertices are not integers here and a row may start
+  // up to one row outside the triangle, so the ranges are checked by row.
+  __device__ __forceinline__ int put(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int slot, int lo,
+                                     int cnt, int &addr, int &x) {
+    x = lo;
+    addr = cy * P.view.w + lo;
+    bool safe = cz1 >= 0x1p-60f && cz2 >= 0x1p-60f && cz1 <= 0x1p60f && cz2 <= 0x1p60f && fabsf(cx2) <= 0x1p59f &&
+                fabsf(cx1 - cx2) <= 0x1p59f;
+    if (span_put<ALPHA>(q, slot, safe, lo, ~make_order(1, gtri, half), cx1, cx2, cz1, cz2, cu1, cu2, g)) return cnt;
+    vis_serial<ALPHA>(P.keys, sg, q, slot, cnt, addr, x);
     return 0;
   }
 
-  __device__ __forceinline__ int emit(const DrawParams &P, const GroupDev *sg, VisQ<ALPHA> &q, int lane, bool &live) {
+  __device__ __forceinline__ int emit(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int slot, int &addr,
+                                      int &x, bool &live) {
     int cnt = 0;
+    // the half's left and right edge; both halves advance alike (start_half1
+    // negates the slopes)
+    const float l = half == 0 ? cx2 : cx1, r = half == 0 ? cx1 : cx2;
+    if (l < xMax && r > xMin) {
+      int lo = f2i(clampf_(l, xMin, xMax));
+      int hi = f2i(floorf(clampf_(r, xMin, xMax)));
+      cnt = hi >= lo ? hi - lo + 1 : 0;
+      if (cnt) cnt = put(P, sg, q, slot, lo, cnt, addr, x);
+    }
+    cx1 += s1; cx2 += s2; cz1 += sz1; cz2 += sz2;
+    if (ALPHA) { cu1 = add2(cu1, su1); cu2 = add2(cu2, su2); }
     if (half == 0) {
-      if (cx2 < xMax && cx1 > xMin) {
-        int lo = f2i(clampf_(cx2, xMin, xMax));
-        int hi = f2i(floorf(clampf_(cx1, xMin, xMax)));
-        cnt = hi >= lo ? hi - lo + 1 : 0;
-        if (cnt) cnt = put(P, sg, q, lane, lo, cnt);
-      }
-      cx1 += s1; cx2 += s2; cz1 += sz1; cz2 += sz2;
-      if (ALPHA) { cu1 = add2(cu1, su1); cu2 = add2(cu2, su2); }
       cy++;
       if ((float)cy > ybound) {
         start_half1();
         live = live_half;
       }
-      return cnt;
+    } else {
+      cy--;
+      live = (float)cy >= ybound;
     }
-    if (cx1 < xMax && cx2 > xMin) {
-      int lo = f2i(clampf_(cx1, xMin, xMax));
-      int hi = f2i(floorf(clampf_(cx2, xMin, xMax)));
-      cnt = hi >= lo ? hi - lo + 1 : 0;
-      if (cnt) cnt = put(P, sg, q, lane, lo, cnt);
-    }
-    cx1 -= s1; cx2 -= s2; cz1 -= sz1; cz2 -= sz2;
-    if (ALPHA) { cu1 = sub2(cu1, su1); cu2 = sub2(cu2, su2); }
-    cy--;
-    live = (float)cy >= ybound;
     return cnt;
   }
 };
 
 template <bool ALPHA>
-__device__ __forceinline__ void raster_tiled_loop(const DrawParams &P, const GroupDev *sg, VisQ<ALPHA> &q, int lane) {
+__device__ __forceinline__ void raster_tiled_loop(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int lane) {
   if (P.ctr[CTR_OVERFLOW]) return;
   uint32_t n = P.ctr[ALPHA ? CTR_UNITS_A : CTR_UNITS];
   const uint32_t per = ALPHA ? claim_size(n, (uint32_t)P.claim_k) : 32u;
@@ -1417,9 +1440,10 @@ __device__ __forceinline__ void raster_tiled_loop(const DrawParams &P, const Gro
         if (lane == 0) atomicOr(&P.ctr[CTR_LIMIT], 1u);
         break;
       }
-      int cnt = 0;
-      if (live) cnt = L.emit(P, sg, q, lane, live);
-      vis_fill<ALPHA>(P, sg, q, lane, cnt, L.pb);
+      RowPair r = {};
+      if (live) r.cnt[0] = L.emit(P, sg, q, lane, r.addr[0], r.x[0], live);
+      if (live) r.cnt[1] = L.emit(P, sg, q, lane + 32, r.addr[1], r.x[1], live);
+      vis_fill<ALPHA>(P, sg, q, lane, r);
     }
   }
 }
@@ -1427,7 +1451,7 @@ __device__ __forceinline__ void raster_tiled_loop(const DrawParams &P, const Gro
 template <bool ALPHA>
 __global__ void __launch_bounds__(128, ALPHA ? 6 : 8) k_raster_tiled(DrawParams P) {
   __shared__ GroupDev sg[64];
-  __shared__ VisQ<ALPHA> qs[4];
+  __shared__ SpanQ<ALPHA> qs[4];
   for (int i = threadIdx.x; i < P.ngroups; i += blockDim.x) sg[i] = P.groups[i];
   __syncthreads();
   raster_tiled_loop<ALPHA>(P, sg, qs[threadIdx.x >> 5], threadIdx.x & 31);
@@ -1437,18 +1461,18 @@ __global__ void __launch_bounds__(128, ALPHA ? 6 : 8) k_raster_tiled(DrawParams 
 // one triangle per warp, its coarse tiles dealt round-robin to the lanes and
 // each lane filling its tiles on its own (slow, same fragments).
 template <bool ALPHA>
-__device__ __forceinline__ void fallback_unit(const DrawParams &P, const GroupDev *sg, VisQ<ALPHA> &q, int lane,
+__device__ __forceinline__ void fallback_unit(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int lane,
                                               uint32_t gt, int tile) {
   TileLane<ALPHA> L;
   bool live = L.init(P, sg, make_uint2(gt, (uint32_t)tile));
   for (int round = 0; live && round < LOOP_LIMIT; round++) {
-    int cnt = L.emit(P, sg, q, lane, live);   // the lane's own record: pixel j is x = lo + j
-    if (cnt) q.b[lane] = L.pb;
-    for (int j = 0; j < cnt; j++) vis_pixel<ALPHA>(P, sg, q, lane, j);
+    int addr = 0, x = 0, cnt = L.emit(P, sg, q, lane, addr, x, live);   // the lane's own slot: pixel j is x + j
+    if (cnt) span_base(q, lane, addr, x);
+    for (int j = 0; j < cnt; j++) vis_pixel<ALPHA>(P, sg, q, lane * 16, j);
   }
 }
 
-__device__ __forceinline__ void fallback_loop(const DrawParams &P, const GroupDev *sg, VisQ<false> &qo, VisQ<true> &qa,
+__device__ __forceinline__ void fallback_loop(const DrawParams &P, const GroupDev *sg, SpanQ<false> &qo, SpanQ<true> &qa,
                                               int lane, int gw, int nw) {
   if (!P.ctr[CTR_OVERFLOW]) return;
   uint32_t n = P.ctr[CTR_LARGE];
@@ -1470,8 +1494,8 @@ __device__ __forceinline__ void fallback_loop(const DrawParams &P, const GroupDe
 
 __global__ void __launch_bounds__(128) k_raster_tiled_fallback(DrawParams P) {
   __shared__ GroupDev sg[64];
-  __shared__ VisQ<false> qo[4];
-  __shared__ VisQ<true> qa[4];
+  __shared__ SpanQ<false> qo[4];
+  __shared__ SpanQ<true> qa[4];
   for (int i = threadIdx.x; i < P.ngroups; i += blockDim.x) sg[i] = P.groups[i];
   __syncthreads();
   int w = threadIdx.x >> 5;
@@ -2208,19 +2232,58 @@ __device__ __forceinline__ int depth_floor_bits(float cz1, float cz2) {
   return __float_as_int(__fmul_rn(r, 1.0f - 0x1p-18f)) + 1;
 }
 
+// The mask texel of drawminalpha.c:86-96 at a pixel's uv (times z) and depth.
+__device__ __forceinline__ bool mask_texel(const GroupDev &G, float u, float v, float tz) {
+  int len = G.alen;
+  float lm1 = (float)(len - 1);
+  int t1 = f2i((u * tz) * lm1);
+  t1 = iabs_(t1) & (len - 1);
+  int t2 = f2i((lm1 * v) * tz);
+  t2 = iabs_(t2) & (len - 1);
+  return __ldg(G.amask + t1 + t2 * len) != 0;
+}
+
+// drawmin.c:71-76 / drawminalpha.c:83-97 for pixel number p of the span at
+// byte offset `off`; its depth is positive and finite, so it orders as its bits.
+// Alpha-tested casters read the texel first: one that already holds a depth
+// <= tz (most of them, behind the opaque casters) skips the mask lookup.
+// Texels only decrease, so any value read bounds the final one.
 template <bool ALPHA>
-struct ShadowQ {
-  float4 a[32];                  // cx2, d, 1/d (0: divide), cz1
-  float4 b[32];                  // cz2, texel address - first pixel number, x - first pixel number,
-                                 // depth floor bits (tiled pass)
-  float4 c[ALPHA ? 32 : 1];      // cu1, cv1, cu2, cv2
-  int g[ALPHA ? 32 : 1];
-  int r2l[32];
-};
+__device__ __forceinline__ void shadow_pixel(float *map, const GroupDev *sg, const SpanQ<ALPHA> &q, int off, int p) {
+  const float4 a = span_at(q.a, off), b = span_at(q.b, off);
+  float *addr = map + (uint32_t)(p + __float_as_int(b.z));
+  float cur = 0.f;
+  if (ALPHA) cur = __ldcg(addr);
+  float t = span_t((float)(p + __float_as_int(b.w)) - a.x, a.y, a.z), omt = 1 - t;
+  float tz = recip_rn(omt * b.x + t * a.w);
+  if (ALPHA) {
+    if (!(cur > tz)) return;
+    const float4 c = span_at(q.c, off);
+    if (!mask_texel(sg[span_at(q.g, off >> 2)], omt * c.z + t * c.x, omt * c.w + t * c.y, tz)) return;
+  }
+  atomicMin((int *)addr, __float_as_int(tz));
+}
+
+// The span in `slot`, drawn by its lane alone with true divisions.
+template <bool ALPHA>
+__device__ __noinline__ void shadow_serial(float *map, const GroupDev *sg, const SpanQ<ALPHA> &q, int slot, int cnt,
+                                           int addr, int x) {
+  const float4 a = q.a[slot], b = q.b[slot];
+  for (int j = 0; j < cnt; j++) {
+    float t = clamp_t(((float)(x + j) - a.x) / a.y), omt = 1 - t;
+    float tz = 1.0f / (omt * b.x + t * a.w);
+    if (tz != tz) continue;
+    if (ALPHA) {
+      const float4 c = q.c[slot];
+      if (!mask_texel(sg[q.g[slot]], omt * c.z + t * c.x, omt * c.w + t * c.y, tz)) continue;
+    }
+    atomic_min_depth(map + (size_t)(addr + j), tz);
+  }
+}
 
 template <bool ALPHA>
 struct ShadowLane {
-  float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);   // second half of the last span record (fill_round stores it)
+  bool safe;     // z_safe of its vertices
   int x1, x2, x3, y1, y2, y3, x4;
   float z1, z2, z3, z4, u1, u2, u3, u4, v1, v2, v3, v4;
   int half, cy, g;
@@ -2228,41 +2291,37 @@ struct ShadowLane {
   float cx1, cx2, cz1, cz2, cu1, cu2, cv1, cv2;
 
   // drawmin.c divides each slope by the row count; one reciprocal serves
-  // them all (quot_by_recip: the same correctly rounded quotients)
-  __device__ __forceinline__ void start_half0() {
-    half = 0;
-    float d = (float)(y2 - y1);
-    float y = span_recip(d);
-    s1 = quot_by_recip((float)(x2 - x1), d, y);
-    s2 = quot_by_recip((float)(x4 - x1), d, y);
+  // them all (the correctly rounded quotients: whole numbers for x, safe z's
+  // differences, see z_safe; u and v checked one by one).  The second half's
+  // slopes are computed with the first's: a lane that reaches its caster's
+  // middle row during the walk then only copies them, instead of stalling the
+  // warp's other lanes for the divisions.
+  float hs1, hs2, hsz1, hsz2, hsu1, hsv1, hsu2, hsv2;
+  __device__ __forceinline__ void slopes() {
+    float d = (float)(y2 - y1), e = (float)(y3 - y2);
+    if (safe) {
+      float y = recip_rn(d), w = recip_rn(e);   // (d or e = 0: that half's slopes are not used)
+      s1 = quot_fast((float)(x2 - x1), d, y); s2 = quot_fast((float)(x4 - x1), d, y);
+      sz1 = quot_fast(z2 - z1, d, y); sz2 = quot_fast(z4 - z1, d, y);
+      hs1 = quot_fast((float)(x3 - x2), e, w); hs2 = quot_fast((float)(x3 - x4), e, w);
+      hsz1 = quot_fast(z3 - z2, e, w); hsz2 = quot_fast(z3 - z4, e, w);
+    } else {
+      s1 = (float)(x2 - x1) / d; s2 = (float)(x4 - x1) / d;
+      sz1 = (z2 - z1) / d; sz2 = (z4 - z1) / d;
+      hs1 = (float)(x3 - x2) / e; hs2 = (float)(x3 - x4) / e;
+      hsz1 = (z3 - z2) / e; hsz2 = (z3 - z4) / e;
+    }
     if (ALPHA) {
+      float y = span_recip(d), w = span_recip(e);
       su1 = quot_by_recip(u2 - u1, d, y); sv1 = quot_by_recip(v2 - v1, d, y);
       su2 = quot_by_recip(u4 - u1, d, y); sv2 = quot_by_recip(v4 - v1, d, y);
+      hsu1 = quot_by_recip(u3 - u2, e, w); hsv1 = quot_by_recip(v3 - v2, e, w);
+      hsu2 = quot_by_recip(u3 - u4, e, w); hsv2 = quot_by_recip(v3 - v4, e, w);
     }
-    sz1 = quot_by_recip(z2 - z1, d, y); sz2 = quot_by_recip(z4 - z1, d, y);
-    cx1 = cx2 = (float)x1; cz1 = cz2 = z1;
-    if (ALPHA) { cu1 = cu2 = u1; cv1 = cv2 = v1; }
     if (s1 < s2) {
       swap_(s1, s2); swap_(sz1, sz2);
       if (ALPHA) { swap_(su1, su2); swap_(sv1, sv2); }
     }
-    cy = y1;
-  }
-  // The second half's slopes are computed with the first's, when the
-  // caster is set up: a lane that reaches its caster's middle row during
-  // the walk then only copies them, instead of stalling the warp's other
-  // lanes for the divisions.
-  float hs1, hs2, hsz1, hsz2, hsu1, hsv1, hsu2, hsv2;
-  __device__ __forceinline__ void half1_slopes() {
-    float d = (float)(y3 - y2);
-    float y = span_recip(d);
-    hs1 = quot_by_recip((float)(x3 - x2), d, y);
-    hs2 = quot_by_recip((float)(x3 - x4), d, y);
-    if (ALPHA) {
-      hsu1 = quot_by_recip(u3 - u2, d, y); hsv1 = quot_by_recip(v3 - v2, d, y);
-      hsu2 = quot_by_recip(u3 - u4, d, y); hsv2 = quot_by_recip(v3 - v4, d, y);
-    }
-    hsz1 = quot_by_recip(z3 - z2, d, y); hsz2 = quot_by_recip(z3 - z4, d, y);
     if (hs1 < hs2) {
       swap_(hs1, hs2); swap_(hsz1, hsz2);
       if (ALPHA) { swap_(hsu1, hsu2); swap_(hsv1, hsv2); }
@@ -2270,6 +2329,12 @@ struct ShadowLane {
     // walked upwards by additions of the negated slopes (see SmallLane)
     hs1 = -hs1; hs2 = -hs2; hsz1 = -hsz1; hsz2 = -hsz2;
     if (ALPHA) { hsu1 = -hsu1; hsv1 = -hsv1; hsu2 = -hsu2; hsv2 = -hsv2; }
+  }
+  __device__ __forceinline__ void start_half0() {
+    half = 0;
+    cx1 = cx2 = (float)x1; cz1 = cz2 = z1;
+    if (ALPHA) { cu1 = cu2 = u1; cv1 = cv2 = v1; }
+    cy = y1;
   }
   __device__ __forceinline__ void start_half1() {
     half = 1;
@@ -2305,7 +2370,9 @@ struct ShadowLane {
   // drawmin.c:49-51 (split vertex) and the first half's slopes, from the
   // sorted vertices
   __device__ __forceinline__ void finish(const V2 uv[3]) {
-    float q = (float)(y2 - y1) / (float)(y3 - y1);
+    float hgt = (float)(y3 - y1);   // (0: one row, the split vertex is not used)
+    float q = quot_fast((float)(y2 - y1), hgt, recip_rn(hgt));
+    safe = z_safe(z1, z2, z3);
     x4 = f2i((float)x1 + q * (float)(x3 - x1));
     z4 = z1 + q * (z3 - z1);
     if (ALPHA) {
@@ -2313,7 +2380,7 @@ struct ShadowLane {
       u4 = u1 + q * (u3 - u1);
       v4 = v1 + q * (v3 - v1);
     }
-    half1_slopes();
+    slopes();
     start_half0();
     left = y3 - y1 + 1;
   }
@@ -2357,7 +2424,6 @@ struct ShadowLane {
   }
 
   int left;      // rows left in this lane's chunk (a whole caster: y3 - y1 + 1)
-  bool serial;   // emit_tile: the span just written needs the true division
 
   // advances one row of the current half
   __device__ __forceinline__ void step() {
@@ -2393,26 +2459,18 @@ struct ShadowLane {
     return true;
   }
 
-  // sets `serial` when the span just written needs the true division (the
-  // caller then draws it with this lane alone)
-  __device__ __forceinline__ int emit(int dim, ShadowQ<ALPHA> &q, int lane, bool &live) {
-    serial = false;
+  // writes the current row's span into `slot`, advances; returns its pixels
+  __device__ __forceinline__ int emit(float *map, int dim, const GroupDev *sg, SpanQ<ALPHA> &q, int slot, int &addr,
+                                      int &x, bool &live) {
     int cnt = 0;
     if (cy >= 0 && cy < dim) {
-      int a0 = half == 0 ? f2i(cx2) : f2i(cx1);
-      int a1 = half == 0 ? f2i(cx1) : f2i(cx2);
-      int lo = a0 < 0 ? 0 : a0, hi = a1 > dim - 1 ? dim - 1 : a1;
+      int lo = max(f2i(half == 0 ? cx2 : cx1), 0), hi = min(f2i(half == 0 ? cx1 : cx2), dim - 1);
       cnt = hi >= lo ? hi - lo + 1 : 0;
-      if (cnt) {
-        float qx, qd, qy;
-        serial = !span_queue_form(cx2, cx1 - cx2, lo, qx, qd, qy);
-        q.a[lane] = make_float4(qx, qd, qy, cz1);
-        pb = make_float4(cz2, __int_as_float(cy * dim + lo), __int_as_float(lo), 0.f);
-        if (serial) q.b[lane] = pb;
-        if (ALPHA) {
-          q.c[lane] = make_float4(cu1, cv1, cu2, cv2);
-          q.g[lane] = g;
-        }
+      x = lo;
+      addr = cy * dim + lo;
+      if (cnt && !span_put<ALPHA>(q, slot, safe, lo, 0u, cx1, cx2, cz1, cz2, V2{cu1, cv1}, V2{cu2, cv2}, g)) {
+        shadow_serial<ALPHA>(map, sg, q, slot, cnt, addr, x);
+        cnt = 0;
       }
     }
     next_row();
@@ -2422,14 +2480,12 @@ struct ShadowLane {
 
   // emit() inside a tile: the current row lies in rows ty0..ty1; its span is
   // clipped to columns tx0..tx1 and written with its texel offset in the
-  // tile and its depth floor.  Then advances to the next row in the tile.
-  // A span whose depth floor lies above every texel it covers (by the
-  // tile's sub-block maxima `smax`) is not queued.
-  __device__ __forceinline__ int emit_tile(ShadowQ<ALPHA> &q, int lane, int tx0, int tx1, int ty0, int ty1,
-                                           const int *smax, bool &live) {
-    int a0 = half == 0 ? f2i(cx2) : f2i(cx1);
-    int a1 = half == 0 ? f2i(cx1) : f2i(cx2);
-    int lo = max(a0, tx0), hi = min(a1, tx1);
+  // tile (row stride TROW) and its depth floor.  Then advances to the next
+  // row in the tile.  A span whose depth floor lies above every texel it
+  // covers (by the tile's sub-block maxima `smax`) is not queued.
+  __device__ __forceinline__ int emit_tile(int *tile, const GroupDev *sg, SpanQ<ALPHA> &q, int slot, int tx0, int tx1,
+                                           int ty0, int ty1, const int *smax, int &addr, int &x, bool &live) {
+    int lo = max(f2i(half == 0 ? cx2 : cx1), tx0), hi = min(f2i(half == 0 ? cx1 : cx2), tx1);
     int cnt = hi >= lo ? hi - lo + 1 : 0;
     int floor_bits = 0;
     if (cnt) {
@@ -2439,18 +2495,12 @@ struct ShadowLane {
       for (int bx = (lo - tx0) >> SUB_LOG; bx <= (hi - tx0) >> SUB_LOG; bx++) m = max(m, row[bx]);
       if (m < floor_bits) cnt = 0;
     }
-    serial = false;
-    if (cnt) {
-      float qx, qd, qy;
-      serial = !span_queue_form(cx2, cx1 - cx2, lo, qx, qd, qy);   // then the caller draws it with this lane alone
-      q.a[lane] = make_float4(qx, qd, qy, cz1);
-      pb = make_float4(cz2, __int_as_float((cy - ty0) * TROW + (lo - tx0)), __int_as_float(lo),
-                       __int_as_float(floor_bits));
-      if (serial) q.b[lane] = pb;
-      if (ALPHA) {
-        q.c[lane] = make_float4(cu1, cv1, cu2, cv2);
-        q.g[lane] = g;
-      }
+    x = lo;
+    addr = (cy - ty0) * TROW + (lo - tx0);
+    if (cnt && !span_put<ALPHA>(q, slot, safe, lo, (uint32_t)floor_bits, cx1, cx2, cz1, cz2, V2{cu1, cv1},
+                                V2{cu2, cv2}, g)) {
+      shadow_serial<ALPHA>(reinterpret_cast<float *>(tile), sg, q, slot, cnt, addr, x);
+      cnt = 0;
     }
     next_row();
     --left;
@@ -2463,47 +2513,8 @@ struct ShadowLane {
   }
 };
 
-// drawmin.c:71-76 / drawminalpha.c:83-97 for pixel number p of span s: the
-// depth tz, or false when nothing is written (NaN depth, alpha discard)
-template <bool ALPHA, bool DIV = false, bool EZ = false>
-__device__ __forceinline__ bool shadow_depth(const GroupDev *sg, const ShadowQ<ALPHA> &q, int s, int p, float4 b,
-                                             float &tz, float cur = 0.f) {
-  const float4 a = q.a[s];
-  float n = (float)(p + __float_as_int(b.z)) - a.x;
-  float t = DIV ? clamp_t(n / a.y) : span_t(n, a.y, a.z);
-  tz = __frcp_rn((1 - t) * b.x + t * a.w);
-  if (tz != tz) return false;
-  if (EZ && !(cur > tz)) return false;
-  if (ALPHA) {
-    const float4 c = q.c[s];
-    const GroupDev &G = sg[q.g[s]];
-    int len = G.alen;
-    float lm1 = (float)(len - 1);
-    int t1 = f2i((((1 - t) * c.z + t * c.x) * tz) * lm1);
-    t1 = iabs_(t1) & (len - 1);
-    int t2 = f2i((lm1 * ((1 - t) * c.w + t * c.y)) * tz);
-    t2 = iabs_(t2) & (len - 1);
-    if (!__ldg(G.amask + t1 + t2 * len)) return false;
-  }
-  return true;
-}
-
-// drawmin.c:71-76 / drawminalpha.c:83-97 for one pixel of span s
-template <bool ALPHA, bool DIV = false>
-__device__ __forceinline__ void shadow_pixel(float *map, const GroupDev *sg, const ShadowQ<ALPHA> &q, int s, int p) {
-  const float4 b = q.b[s];
-  float *addr = map + (size_t)(p + __float_as_int(b.y));
-  // alpha-tested casters read the texel first: one that already holds a
-  // depth <= tz (most of them, behind the opaque casters) skips the mask
-  // lookup.  Texels only decrease, so any value read bounds the final one.
-  float cur = 0.f;
-  if (ALPHA) cur = __ldcg(addr);
-  float tz;
-  if (shadow_depth<ALPHA, DIV, ALPHA>(sg, q, s, p, b, tz, cur)) atomic_min_depth(addr, tz);
-}
-
 template <bool ALPHA>
-__device__ __forceinline__ void shadow_warp_loop(const ShadowParams &S, const GroupDev *sg, ShadowQ<ALPHA> &q, int lane,
+__device__ __forceinline__ void shadow_warp_loop(const ShadowParams &S, const GroupDev *sg, SpanQ<ALPHA> &q, int lane,
                                                  int ctr_list, int ctr_work) {
   // work items: row chunks of the casters when S.items is given, else casters
   const bool chunked = S.items != nullptr;
@@ -2533,15 +2544,10 @@ __device__ __forceinline__ void shadow_warp_loop(const ShadowParams &S, const Gr
         if (lane == 0) atomicOr(&S.ctr[CTR_LIMIT], 1u);
         break;
       }
-      int cnt = 0;
-      if (live) {
-        cnt = L.emit(dim, q, lane, live);
-        if (L.serial) {   // a span the queue cannot take: this lane draws it
-          for (int j = 0; j < cnt; j++) shadow_pixel<ALPHA, true>(S.map, sg, q, lane, j);
-          cnt = 0;
-        }
-      }
-      fill_round(q, lane, cnt, L.pb, [&](int s, int p) { shadow_pixel<ALPHA>(S.map, sg, q, s, p); });
+      RowPair r = {};
+      if (live) r.cnt[0] = L.emit(S.map, dim, sg, q, lane, r.addr[0], r.x[0], live);
+      if (live) r.cnt[1] = L.emit(S.map, dim, sg, q, lane + 32, r.addr[1], r.x[1], live);
+      fill_rows<false>(q, lane, r, [&](int off, int p) { shadow_pixel<ALPHA>(S.map, sg, q, off, p); }, [](int) {});
     }
   }
 }
@@ -2552,7 +2558,7 @@ __device__ __forceinline__ void shadow_warp_loop(const ShadowParams &S, const Gr
 template <bool ALPHA>
 __global__ void __launch_bounds__(128, ALPHA ? 7 : 9) k_shadow_raster(ShadowParams S) {
   __shared__ GroupDev sg[64];
-  __shared__ ShadowQ<ALPHA> qs[4];
+  __shared__ SpanQ<ALPHA> qs[4];
   for (int i = threadIdx.x; i < S.ngroups; i += blockDim.x) sg[i] = S.groups[i];
   __syncthreads();
   int w = threadIdx.x >> 5, lane = threadIdx.x & 31;

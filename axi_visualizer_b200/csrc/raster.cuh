@@ -117,19 +117,6 @@ __device__ __forceinline__ float span_recip(float d) {
   float a = fabsf(d);
   return (a >= 8.6736174e-19f && a <= 1.1529215e18f) ? __frcp_rn(d) : 0.f;
 }
-// y of span_recip(d) when, in addition, every quotient (ax - cx2) / d of the
-// span's pixels (integer ax >= lo >= 0) can take the reciprocal path: then
-// |ax - cx2| <= 2^60 and it is 0 or >= 2^-60 (for |cx2| >= 2^-36 the exact
-// difference is a multiple of ulp(cx2) >= 2^-59; for smaller cx2 it is
-// either cx2 itself, when ax = 0 and cx2 = 0, or at least 1 - 2^-36).
-// Returns 0 when a pixel might need the true division.
-__device__ __forceinline__ float span_recip_exact(float d, float cx2, int lo) {
-  float y = span_recip(d);
-  float a = fabsf(cx2);
-  bool ok = a <= 0x1p59f && (a >= 0x1p-36f || cx2 == 0.f || lo > 0);
-  return ok ? y : 0.f;
-}
-
 // The quotient of quot_by_recip when the operands are known to be in range.
 __device__ __forceinline__ float quot_fast(float n, float d, float y) {
   float q = __fmul_rn(n, y);
@@ -137,34 +124,26 @@ __device__ __forceinline__ float quot_fast(float n, float d, float y) {
   return __fmaf_rn(r, y, q);
 }
 
-// t = clamp(n / d, 0, 1) of a pixel of a span queued by span_queue_form.
-// The operands are in range there (finite, d and y nonzero), so the
-// quotient is never NaN and the clamp needs no NaN rule.
+// t = clamp(n / d, 0, 1) of a pixel of a queued span.  The operands are in
+// range there (finite, d and y nonzero), so the quotient is never NaN and
+// the last step of quot_fast can saturate to [0, 1] itself.
 __device__ __forceinline__ float span_t(float n, float d, float y) {
-  return fmaxf(0.f, fminf(1.f, quot_fast(n, d, y)));
+  float q = __fmul_rn(n, y);
+  float r = __fmaf_rn(-d, q, n);
+  float t;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(t) : "f"(r), "f"(y), "f"(q));
+  return t;
 }
 
-// The (cx2, d, y) a span with first pixel lo is queued with, so that every
-// pixel x of it takes t = span_t(x - cx2, d, y).  Usually (cx2, d, RN(1/d)).
-// d = cx1 - cx2 = +-0 means cx1 and cx2 are equal (or both zero), so the
-// span is the one pixel lo: its n / d is an infinity of sign sign(n) xor
-// sign(d), clamped to 1 or 0, or NaN for n = 0, clamped to 1; that t is
-// fixed here as cx2 = lo - 1 (t = 1) or lo + 1 (t = 0) with d = y = 1.
-// Returns false when a pixel might need the true division (a reciprocal out
-// of the safe range with d != 0, which real scenes almost never produce):
-// the span's own lane then draws it with the true cx2 and d.
-__device__ __forceinline__ bool span_queue_form(float cx2, float d, int lo, float &qx, float &qd, float &qy) {
-  qx = cx2;
-  qd = d;
-  qy = span_recip_exact(d, cx2, lo);
-  if (qy != 0.f) return true;
-  if (d != 0.f) return false;
-  float n = (float)lo - cx2;
-  bool one = n == 0.f || ((__float_as_uint(n) ^ __float_as_uint(d)) & 0x80000000u) == 0u;
-  qx = (float)lo - (one ? 1.f : -1.f);
-  qd = 1.f;
-  qy = 1.f;
-  return true;
+// RN(1 / v) for 2^-61 <= |v| < 2^62: the approximate reciprocal (within one
+// ulp) and one residual step, e = 1 - v r, r + r e, which Markstein's paper
+// shows to round correctly except perhaps for isolated mantissas; compared
+// with __frcp_rn over every mantissa, both signs and all these exponents it
+// has none.  Three instructions, no branch, against about ten.
+__device__ __forceinline__ float recip_rn(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return __fmaf_rn(r, __fmaf_rn(-v, r, 1.0f), r);
 }
 
 __device__ __forceinline__ float quot_by_recip(float n, float d, float y) {

@@ -213,17 +213,20 @@ __global__ void __launch_bounds__(256) k_shadow_sort(ShadowParams S) {
   }
 }
 
-// One texel of a tile: the depth-floor test, then drawmin.c's depth and the
-// minimum in shared memory (the per-caster path's atomic_min_depth).
-template <bool ALPHA, bool DIV = false>
-__device__ __forceinline__ void tile_pixel(int *tile, const GroupDev *sg, const ShadowQ<ALPHA> &q, int s, int p) {
-  const float4 b = q.b[s];
-  int off = p + __float_as_int(b.y);
-  if (tile[off] < __float_as_int(b.w)) return;
-  float tz;
-  if (!shadow_depth<ALPHA, DIV>(sg, q, s, p, b, tz)) return;
-  if (tz >= 0.f) atomicMin(tile + off, __float_as_int(tz));
-  else atomicMax((unsigned int *)(tile + off), __float_as_uint(tz));
+// One texel of a tile: the depth-floor test, then the depth as shadow_pixel
+// computes it and the minimum in shared memory.
+template <bool ALPHA>
+__device__ __forceinline__ void tile_pixel(int *tile, const GroupDev *sg, const SpanQ<ALPHA> &q, int off, int p) {
+  const float4 a = span_at(q.a, off), b = span_at(q.b, off);
+  int *texel = tile + (p + __float_as_int(b.z));
+  if (*texel < __float_as_int(b.y)) return;
+  float t = span_t((float)(p + __float_as_int(b.w)) - a.x, a.y, a.z), omt = 1 - t;
+  float tz = recip_rn(omt * b.x + t * a.w);
+  if (ALPHA) {
+    const float4 c = span_at(q.c, off);
+    if (!mask_texel(sg[span_at(q.g, off >> 2)], omt * c.z + t * c.x, omt * c.w + t * c.y, tz)) return;
+  }
+  atomicMin(texel, __float_as_int(tz));
 }
 
 // Upper bounds of the texel bits of each 8 x 8 sub-block of the tile, as
@@ -282,7 +285,7 @@ __device__ __forceinline__ bool unit_hidden(const ShadowParams &S, uint32_t r, c
 // per lane, rows and spans clipped to the tile.
 template <bool ALPHA>
 __device__ __forceinline__ void tile_units(const ShadowParams &S, const GroupDev *sg, int *tile, int *smax,
-                                           uint32_t *ready, ShadowQ<ALPHA> &q, int lane, uint32_t u0, uint32_t n,
+                                           uint32_t *ready, SpanQ<ALPHA> &q, int lane, uint32_t u0, uint32_t n,
                                            uint32_t *claim, int tx0, int tx1, int ty0, int ty1) {
   const unsigned below = (1u << lane) - 1u;
   int have = 0;
@@ -325,15 +328,10 @@ __device__ __forceinline__ void tile_units(const ShadowParams &S, const GroupDev
         if (lane == 0) atomicOr(&S.ctr[CTR_LIMIT], 1u);
         break;
       }
-      int cnt = 0;
-      if (live) {
-        cnt = L.emit_tile(q, lane, tx0, tx1, ty0, ty1, smax, live);
-        if (L.serial) {   // a span the queue cannot take: this lane draws it
-          for (int j = 0; j < cnt; j++) tile_pixel<ALPHA, true>(tile, sg, q, lane, j);
-          cnt = 0;
-        }
-      }
-      fill_round(q, lane, cnt, L.pb, [&](int s, int p) { tile_pixel<ALPHA>(tile, sg, q, s, p); });
+      RowPair r = {};
+      if (live) r.cnt[0] = L.emit_tile(tile, sg, q, lane, tx0, tx1, ty0, ty1, smax, r.addr[0], r.x[0], live);
+      if (live) r.cnt[1] = L.emit_tile(tile, sg, q, lane + 32, tx0, tx1, ty0, ty1, smax, r.addr[1], r.x[1], live);
+      fill_rows<false>(q, lane, r, [&](int off, int p) { tile_pixel<ALPHA>(tile, sg, q, off, p); }, [](int) {});
     }
   }
 }
@@ -348,7 +346,7 @@ template <bool ALPHA>
 __global__ void __launch_bounds__(TILE_THREADS, ALPHA ? 6 : 8) k_shadow_tiles(ShadowParams S) {
   __shared__ GroupDev sg[64];
   __shared__ int tile[STILE * TROW];
-  __shared__ ShadowQ<ALPHA> qs[TILE_THREADS / 32];
+  __shared__ SpanQ<ALPHA> qs[TILE_THREADS / 32];
   __shared__ int smax[TILE_THREADS / 32][SUBS * SUBS];
   __shared__ uint32_t ready[TILE_THREADS / 32][64];
   __shared__ uint32_t s_k;
