@@ -701,17 +701,25 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_setup(DrawParams P) {
 // ------------------------------------------------------------ span queue
 
 // One round of a warp: every lane queues the spans of its item's next two
-// rows (row k of lane l in slot l + 32 k), structure of arrays in shared
+// rows (row k of lane l in slot l + SLOT2 k), structure of arrays in shared
 // memory, and the warp then fills their pixels cooperatively.  Two rows a
 // round, not one: numbering a round's pixels costs the same for both, and
 // the last, partly empty window of 32 pixels comes half as often.  Spans of
 // tall thin triangles (two pixels a row) cost the most per row, and gain most.
+// What bounds it is instruction issue: with the pixel body that span_put's
+// ranges allow (no division, no NaN or sign case), warp instructions of the
+// 1080p / 1.04M-triangle frame went 208 -> 145M and 123 -> 82M (opaque casters
+// of the two cascades), 125 -> 82M (opaque small triangles), 92 -> 72M
+// (alpha-tested), 49 -> 40M and 29 -> 18M (tile units), frame 1051 -> 900 us.
+// A lane's second slot lies 64 bytes off its first in the banks, so that a
+// window's reads (both rows of about four neighbouring lanes) do not collide.
+constexpr int SLOT2 = 36, SLOTS = SLOT2 + 32;
 template <bool ALPHA>
 struct SpanQ {
-  float4 a[64];                  // cx2, d = cx1 - cx2, RN(1 / d), cz1
-  float4 b[64];                  // cz2, ~order (views), address and x of pixel number 0
-  float4 c[ALPHA ? 64 : 1];      // u, v (times z) of the first end, of the second
-  int g[ALPHA ? 64 : 1];
+  float4 a[SLOTS];               // cx2, d = cx1 - cx2, RN(1 / d), cz1
+  float4 b[SLOTS];               // cz2, ~order (views), address and x of pixel number 0
+  float4 c[ALPHA ? SLOTS : 1];   // u, v (times z) of the first end, of the second
+  int g[ALPHA ? SLOTS : 1];
   int at[64];                    // rank among the round's non-empty spans -> byte offset of its a and b
 };
 
@@ -797,8 +805,8 @@ __device__ __forceinline__ void fill_rows(Q &q, int lane, const RowPair &r, F &&
     q.at[rank++] = lane * 16;
   }
   if (c1) {
-    span_base(q, lane + 32, r.addr[1] - pre1, r.x[1] - pre1);
-    q.at[rank] = (lane + 32) * 16;
+    span_base(q, lane + SLOT2, r.addr[1] - pre1, r.x[1] - pre1);
+    q.at[rank] = (lane + SLOT2) * 16;
   }
   __syncwarp();
   uint32_t s0 = c0 ? (uint32_t)pre0 : 0x80000000u, s1 = c1 ? (uint32_t)pre1 : 0x80000000u;
@@ -1117,7 +1125,7 @@ __device__ __forceinline__ void raster_small_loop(const DrawParams &P, const Gro
       }
       RowPair r = {};
       if (live) r.cnt[0] = L.emit(P, sg, q, lane, r.addr[0], r.x[0], live);
-      if (live) r.cnt[1] = L.emit(P, sg, q, lane + 32, r.addr[1], r.x[1], live);
+      if (live) r.cnt[1] = L.emit(P, sg, q, lane + SLOT2, r.addr[1], r.x[1], live);
       vis_fill<ALPHA, true>(P, sg, q, lane, r);
     }
   }
@@ -1442,7 +1450,7 @@ __device__ __forceinline__ void raster_tiled_loop(const DrawParams &P, const Gro
       }
       RowPair r = {};
       if (live) r.cnt[0] = L.emit(P, sg, q, lane, r.addr[0], r.x[0], live);
-      if (live) r.cnt[1] = L.emit(P, sg, q, lane + 32, r.addr[1], r.x[1], live);
+      if (live) r.cnt[1] = L.emit(P, sg, q, lane + SLOT2, r.addr[1], r.x[1], live);
       vis_fill<ALPHA>(P, sg, q, lane, r);
     }
   }
@@ -2243,25 +2251,43 @@ __device__ __forceinline__ bool mask_texel(const GroupDev &G, float u, float v, 
   return __ldg(G.amask + t1 + t2 * len) != 0;
 }
 
-// drawmin.c:71-76 / drawminalpha.c:83-97 for pixel number p of the span at
-// byte offset `off`; its depth is positive and finite, so it orders as its bits.
-// Alpha-tested casters read the texel first: one that already holds a depth
-// <= tz (most of them, behind the opaque casters) skips the mask lookup.
-// Texels only decrease, so any value read bounds the final one.
-template <bool ALPHA>
-__device__ __forceinline__ void shadow_pixel(float *map, const GroupDev *sg, const SpanQ<ALPHA> &q, int off, int p) {
+// drawmin.c:71-76 for pixel number p of the span at byte offset `off`; its
+// depth is positive and finite, so it orders as its bits.
+__device__ __forceinline__ void shadow_pixel(float *map, const SpanQ<false> &q, int off, int p) {
   const float4 a = span_at(q.a, off), b = span_at(q.b, off);
-  float *addr = map + (uint32_t)(p + __float_as_int(b.z));
-  float cur = 0.f;
-  if (ALPHA) cur = __ldcg(addr);
-  float t = span_t((float)(p + __float_as_int(b.w)) - a.x, a.y, a.z), omt = 1 - t;
-  float tz = recip_rn(omt * b.x + t * a.w);
-  if (ALPHA) {
-    if (!(cur > tz)) return;
-    const float4 c = span_at(q.c, off);
-    if (!mask_texel(sg[span_at(q.g, off >> 2)], omt * c.z + t * c.x, omt * c.w + t * c.y, tz)) return;
-  }
-  atomicMin((int *)addr, __float_as_int(tz));
+  float t = span_t((float)(p + __float_as_int(b.w)) - a.x, a.y, a.z);
+  float tz = recip_rn((1 - t) * b.x + t * a.w);
+  atomicMin((int *)map + (uint32_t)(p + __float_as_int(b.z)), __float_as_int(tz));
+}
+
+// drawminalpha.c:83-97 in two stages: the first reads the texel, the second
+// drops the pixel when the texel already holds a depth <= its own (most of
+// them, behind the opaque casters) and looks the mask up otherwise.  Texels only
+// decrease, so any value read bounds the final one.  Staged, since the read
+// was what the kernel waited for (5.8 long-scoreboard cycles per issue): the
+// 4K / 2.9M-triangle frame 2267 -> 2245 us, 1080p / 1.04M 887 -> 881 us.
+struct CasterFrag {
+  float tz, cur, t;
+  int off;
+  uint32_t addr;
+};
+__device__ __forceinline__ CasterFrag caster_first(const float *map, const SpanQ<true> &q, int off, int p) {
+  const float4 a = span_at(q.a, off), b = span_at(q.b, off);
+  CasterFrag f;
+  f.addr = (uint32_t)(p + __float_as_int(b.z));
+  f.cur = __ldcg(map + f.addr);
+  f.t = span_t((float)(p + __float_as_int(b.w)) - a.x, a.y, a.z);
+  f.tz = recip_rn((1 - f.t) * b.x + f.t * a.w);
+  f.off = off;
+  return f;
+}
+__device__ __forceinline__ void caster_second(float *map, const GroupDev *sg, const SpanQ<true> &q,
+                                              const CasterFrag &f) {
+  if (!(f.cur > f.tz)) return;
+  const float4 c = span_at(q.c, f.off);
+  float omt = 1 - f.t;
+  if (!mask_texel(sg[span_at(q.g, f.off >> 2)], omt * c.z + f.t * c.x, omt * c.w + f.t * c.y, f.tz)) return;
+  atomicMin((int *)map + f.addr, __float_as_int(f.tz));
 }
 
 // The span in `slot`, drawn by its lane alone with true divisions.
@@ -2546,8 +2572,12 @@ __device__ __forceinline__ void shadow_warp_loop(const ShadowParams &S, const Gr
       }
       RowPair r = {};
       if (live) r.cnt[0] = L.emit(S.map, dim, sg, q, lane, r.addr[0], r.x[0], live);
-      if (live) r.cnt[1] = L.emit(S.map, dim, sg, q, lane + 32, r.addr[1], r.x[1], live);
-      fill_rows<false>(q, lane, r, [&](int off, int p) { shadow_pixel<ALPHA>(S.map, sg, q, off, p); }, [](int) {});
+      if (live) r.cnt[1] = L.emit(S.map, dim, sg, q, lane + SLOT2, r.addr[1], r.x[1], live);
+      if constexpr (ALPHA)
+        fill_rows<true>(q, lane, r, [&](int off, int p) { return caster_first(S.map, q, off, p); },
+                        [&](const CasterFrag &f) { caster_second(S.map, sg, q, f); });
+      else
+        fill_rows<false>(q, lane, r, [&](int off, int p) { shadow_pixel(S.map, q, off, p); }, [](int) {});
     }
   }
 }

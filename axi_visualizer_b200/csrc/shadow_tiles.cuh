@@ -330,7 +330,7 @@ __device__ __forceinline__ void tile_units(const ShadowParams &S, const GroupDev
       }
       RowPair r = {};
       if (live) r.cnt[0] = L.emit_tile(tile, sg, q, lane, tx0, tx1, ty0, ty1, smax, r.addr[0], r.x[0], live);
-      if (live) r.cnt[1] = L.emit_tile(tile, sg, q, lane + 32, tx0, tx1, ty0, ty1, smax, r.addr[1], r.x[1], live);
+      if (live) r.cnt[1] = L.emit_tile(tile, sg, q, lane + SLOT2, tx0, tx1, ty0, ty1, smax, r.addr[1], r.x[1], live);
       fill_rows<false>(q, lane, r, [&](int off, int p) { tile_pixel<ALPHA>(tile, sg, q, off, p); }, [](int) {});
     }
   }
