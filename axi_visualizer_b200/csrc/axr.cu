@@ -1016,7 +1016,7 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
   P.units = c->units; P.ctr = c->ctr;
   P.cap_list = c->cap_list; P.cap_units = c->cap_units;
   P.min_chunk = c->min_chunk;
-  P.claim_k = 2;
+  P.claim_k = 1;
   P.mipc = c->mipc;
   long npix = (long)c->w * c->h;
   cudaStream_t s = c->stream;
@@ -1409,7 +1409,7 @@ int axr_shadow_map(axr_ctx *c, int i, const uint8_t *cast, const int32_t *flags,
   memcpy(S.sh.vv, sm.vv, sizeof sm.vv);
   S.map = sm.map; S.bias = bias; S.list = sm.list; S.cap_list = sm.cap; S.ctr = sm.ctr;
   S.min_chunk = c->min_chunk;
-  S.claim_k = 2;
+  S.claim_k = 1;
   const size_t nt = (size_t)sm.ntx * sm.ntx;
   if (tiled) {
     S.rec = sm.rec;

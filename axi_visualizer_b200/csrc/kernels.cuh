@@ -94,21 +94,25 @@ constexpr int MIN_CHUNK = 12;   // default of DrawParams::min_chunk
 constexpr int CHUNK_BITS = 3;   // work item = list position << CHUNK_BITS | chunk
 constexpr int MAX_CHUNKS = 1 << CHUNK_BITS;
 __device__ __forceinline__ int small_rows(int y1, int y3) { return y3 - y1 + 2; }
-// Items a warp claims at a time in a persistent loop over n work items:
-// one per lane, unless that leaves warps of the launch without work (short
-// queues: the alpha-tested triangles and casters, the large triangles);
-// then fewer, so that every warp gets about `k` claims.  The value is the
-// same for every warp.  On the 1080p scene this took the alpha-tested
-// tiled raster from 133 to 100 us and the alpha casters from 103 to 92 us;
-// the opaque rasterizers stay at 32 (fewer per claim made them slower).
+// Items a warp claims at a time in a persistent loop over n work items: one
+// per lane, unless that leaves warps of the launch without work (short
+// queues); then fewer, so that every warp gets about one claim (k = 1), but at
+// least `least`.  The value is the same for every warp.  Fewer items a claim
+// idle lanes in the row phase, which costs issue slots that other kernels on
+// the GPU could use; more items make one warp's chain of rows and pixels the
+// length of the kernel.  One claim a warp and 8 items, against two claims and
+// any number (alpha-tested queues, casters) or always 32 (opaque): 640x480 /
+// 24k triangles alone 225 -> 183 us, 88 -> 77 us among other frames; 720p /
+// 300k 336 -> 316 and 1080p / 1.04M 886 -> 869 among others (alone 970 -> 990).
 // k = 0: always 32 -- the batched launches, whose warps move on to the
 // next view's queue when one runs dry, so no warp idles.
-__device__ __forceinline__ uint32_t claim_size(uint32_t n, uint32_t k) {
+__device__ __forceinline__ uint32_t claim_size(uint32_t n, uint32_t k, uint32_t least) {
   if (k == 0) return 32u;
   uint32_t nw = gridDim.x * (blockDim.x >> 5) * k;
   uint32_t per = (n + nw - 1) / nw;
-  return per < 1u ? 1u : (per > 32u ? 32u : per);
+  return per < least ? least : (per > 32u ? 32u : per);
 }
+constexpr uint32_t CLAIM_LEAST = 8;   // of the rasterizers
 
 __device__ __forceinline__ int chunk_len(int rows, int min_chunk) {
   int c = (rows + MAX_CHUNKS - 1) / MAX_CHUNKS;
@@ -1104,7 +1108,7 @@ template <bool ALPHA>
 __device__ __forceinline__ void raster_small_loop(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int lane) {
   uint32_t n = P.ctr[ALPHA ? CTR_ITEMS_A : CTR_ITEMS];
   uint32_t cap_items = P.cap_list * MAX_CHUNKS;
-  const uint32_t per = ALPHA ? claim_size(n, (uint32_t)P.claim_k) : 32u;
+  const uint32_t per = claim_size(n, (uint32_t)P.claim_k, CLAIM_LEAST);
   while (true) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(&P.ctr[ALPHA ? CTR_WORK_SMALL_A : CTR_WORK_SMALL], per);
@@ -1205,7 +1209,7 @@ __device__ __forceinline__ void coarse_walk(const float sx[3], const float sy[3]
 __device__ __forceinline__ void coarse_loop(const DrawParams &P, const GroupDev *sg, int lane) {
   uint32_t n = P.ctr[CTR_LARGE];
   int wc = P.view.w / TILE, hc = P.view.h / TILE;
-  const uint32_t per = claim_size(n, P.claim_k > 0 ? 1u : 0u);
+  const uint32_t per = claim_size(n, (uint32_t)P.claim_k, 1u);
   while (true) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(&P.ctr[CTR_WORK_LARGE], per);
@@ -1431,7 +1435,7 @@ template <bool ALPHA>
 __device__ __forceinline__ void raster_tiled_loop(const DrawParams &P, const GroupDev *sg, SpanQ<ALPHA> &q, int lane) {
   if (P.ctr[CTR_OVERFLOW]) return;
   uint32_t n = P.ctr[ALPHA ? CTR_UNITS_A : CTR_UNITS];
-  const uint32_t per = ALPHA ? claim_size(n, (uint32_t)P.claim_k) : 32u;
+  const uint32_t per = claim_size(n, (uint32_t)P.claim_k, CLAIM_LEAST);
   while (true) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(&P.ctr[ALPHA ? CTR_WORK_UNITS_A : CTR_WORK_UNITS], per);
@@ -2547,7 +2551,7 @@ __device__ __forceinline__ void shadow_warp_loop(const ShadowParams &S, const Gr
   uint32_t n = chunked ? S.ctr[ALPHA ? CTR_SH_ITEMS_A : CTR_SH_ITEMS] : S.ctr[ctr_list];
   uint32_t cap_items = S.cap_list * MAX_CHUNKS;
   int dim = S.sh.dim;
-  const uint32_t per = claim_size(n, (uint32_t)S.claim_k);
+  const uint32_t per = claim_size(n, (uint32_t)S.claim_k, CLAIM_LEAST);
   while (true) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(&S.ctr[ctr_work], per);
