@@ -14,7 +14,7 @@
 //                  (triangle, tile) units with warp-scan offsets
 //   k_raster_tiled persistent over units: per-tile restart of the tiled
 //                  `draw` (Templates.py:93-185), same span queue
-//   k_shade        per pixel: decode the winner, replay its row interpolants
+//   k_shade        per 16 x 16 tile: decode the winners, replay their row interpolants
 //                  and shade once (bilinear/trilinear, alpha, shadow)
 // The packed key makes the result independent of scheduling: smallest depth
 // wins, equal depths go to the later fragment of the reference's serial
@@ -43,8 +43,6 @@ struct DrawParams {
   uint32_t cap_list, cap_units;
   int min_chunk;         // rows per small-triangle work item (at least; tuning knob)
   int claim_k;           // claim_size's k for the short queues (0: 32 items per claim)
-  float2 *mipc;          // per triangle of a mip group: (mip fraction, mip level), written by
-                         // the setup, read by the shade; null: the shade computes them
 };
 
 enum {
@@ -653,19 +651,6 @@ __device__ __forceinline__ void setup_phase(const DrawParams &P, const GroupDev 
         cls = project_persp(G, t - G.tri_base, P.view, sx, sy, sz);
         alpha = (G.flags & F_ALPHA) != 0;
         iy0 = f2i(sy[0]); iy1 = f2i(sy[1]); iy2 = f2i(sy[2]);
-        if (P.mipc && cls == 2 && (G.flags & F_MIP)) {
-          // a large triangle's mip level, once here instead of once per
-          // shaded (winner, row) pair; it does not depend on the vertex order
-          Attr<false> a[3];
-          int ix[3], iy[3];
-#pragma unroll
-          for (int k = 0; k < 3; k++) {
-            a[k] = a_load<false>(G, t - G.tri_base, k, sz[k]);
-            ix[k] = f2i(sx[k]); iy[k] = f2i(sy[k]);
-          }
-          MipSel m = mip_setup<false>(a, sz, cls == 1, ix, iy, sx, sy, G.tex_size, G.mip_bias);
-          P.mipc[t] = make_float2(m.fmip, (float)m.mip);
-        }
       }
     }
     unsigned ms = __ballot_sync(FULL, cls == 1 && !alpha), ma = __ballot_sync(FULL, cls == 1 && alpha);
@@ -1545,23 +1530,40 @@ __device__ __forceinline__ float shadow_light(const DrawParams &P, V3 p) {
 template <class A>
 __device__ __forceinline__ void swap_(A &a, A &b) { A t = a; a = b; b = t; }
 
-// The interpolants of winner `ord` on row cy: triangle set-up, mip level and
-// the row accumulation (small triangles from their first row, large ones
-// from the tile's first row), as the rasterizer walked them.
+// One edge chain of a triangle half on some row: x, 1/depth and the attributes
+// (times 1/depth).
+struct EdgeState {
+  float cx, cz;
+  Attr<true> c;
+};
+constexpr int EDGE_WORDS = sizeof(EdgeState) / 4;
+// A (winner, row) pair's two edge chains (an odd number of words: pairs in
+// different banks)
 struct RowState {
-  float cx1, cx2, cz1, cz2;
-  Attr<true> c1, c2;
+  EdgeState e[2];
+  float pad_;
+};
+// A winner (triangle half) in one tile: its edge chains' first states there,
+// their steps a row (negated for the half walked upwards: a - b is a + (-b)
+// exactly), and the row they start from.
+struct WinnerState {
+  EdgeState start[2], step[2];
+  int y0;
+};
+// What its pixels need of the winner itself
+struct WinnerConst {
   float fmip;
   int mip, g;
   V3 tan, bit;   // F_NORMAL: the triangle's tangent frame
 };
 
 // shader_setup of the normal-mapped sources (av_draw_normmap.c:24-38): the
-// tangent frame from the sorted vertices' uv and position divided by z
+// tangent frame from the sorted vertices' uv and position (times z) divided by z
 // (before the round trip multiplies them back)
-__device__ __noinline__ void normal_frame(const Attr<true> a[3], const float z[3], V3 &tan, V3 &bit) {
+__device__ __forceinline__ void normal_frame(const Attr<false> a[3], const V3 p[3], const float z[3], V3 &tan,
+                                             V3 &bit) {
   V2 uv1 = div2(a[0].uv, z[0]), uv2 = div2(a[1].uv, z[1]), uv3 = div2(a[2].uv, z[2]);
-  V3 p1 = div3(a[0].p, z[0]), p2 = div3(a[1].p, z[1]), p3 = div3(a[2].p, z[2]);
+  V3 p1 = div3(p[0], z[0]), p2 = div3(p[1], z[1]), p3 = div3(p[2], z[2]);
   V2 dUV1 = sub2(uv2, uv1), dUV2 = sub2(uv3, uv1);
   V3 dPos1 = sub3(p2, p1), dPos2 = sub3(p3, p1);
   float rdet = 1.f / (dUV1.x * dUV2.y - dUV1.y * dUV2.x);
@@ -1569,166 +1571,127 @@ __device__ __noinline__ void normal_frame(const Attr<true> a[3], const float z[3
   bit = fast_normalize(mul3(sub3(mul3(dPos2, dUV1.x), mul3(dPos1, dUV2.x)), rdet));
 }
 
-// Replays `steps` rows of the two edge chains (add: downwards, else upwards)
-// and stores them in st: edge 0 the first chain (cx1, cz1, c1), edge 1 the
-// second (cx2, cz2, c2), edge 2 both.  The chains are independent sequences
-// of rounded additions, so two threads can each replay one of them and the
-// results are those of one thread replaying both.
-__device__ __forceinline__ void replay_edges(int edge, int steps, bool add, float cx1, float cx2, float cz1, float cz2,
-                                             Attr<true> c1, Attr<true> c2, float s1, float s2, float sz1, float sz2,
-                                             const Attr<true> &sa1, const Attr<true> &sa2, RowState &st) {
-  if (edge == 2) {
-    if (add) {
-      for (int r = 0; r < steps; r++) {
-        cx1 += s1; cx2 += s2; cz1 += sz1; cz2 += sz2; c1 = a_add(c1, sa1); c2 = a_add(c2, sa2);
-      }
-    } else {
-      for (int r = 0; r < steps; r++) {
-        cx1 -= s1; cx2 -= s2; cz1 -= sz1; cz2 -= sz2; c1 = a_sub(c1, sa1); c2 = a_sub(c2, sa2);
-      }
-    }
-    st.cx1 = cx1; st.cx2 = cx2; st.cz1 = cz1; st.cz2 = cz2;
-    st.c1 = c1; st.c2 = c2;
-    return;
-  }
-  const bool e2 = edge != 0;
-  float cx = e2 ? cx2 : cx1, cz = e2 ? cz2 : cz1, s = e2 ? s2 : s1, sz = e2 ? sz2 : sz1;
-  Attr<true> c = e2 ? c2 : c1;
-  const Attr<true> &sa = e2 ? sa2 : sa1;
-  if (add) {
-    for (int r = 0; r < steps; r++) { cx += s; cz += sz; c = a_add(c, sa); }
-  } else {
-    for (int r = 0; r < steps; r++) { cx -= s; cz -= sz; c = a_sub(c, sa); }
-  }
-  if (e2) { st.cx2 = cx; st.cz2 = cz; st.c2 = c; }
-  else { st.cx1 = cx; st.cz1 = cz; st.c1 = c; }
-}
-
-// The row state of winner `ord` on row cy: the edge chain(s) `edge` selects
-// (see replay_edges) and, for edge 0 or 2, the mip level, group and (NRM,
-// F_NORMAL groups) the tangent frame.  NRM = false: draws without
-// normal-mapped groups, whose shade then carries none of that code.
-template <bool NRM = true>
-__device__ __forceinline__ void shade_row_edge(const DrawParams &P, const GroupDev *sg, uint32_t ord, int cy, int edge,
-                                               RowState &st) {
-  uint32_t o = ord - 1;
-  int phase = (int)(o >> 31);
-  uint32_t gtri = (o >> 1) & 0x3fffffffu;
-  int half = (int)(o & 1);
-  int g = find_group(sg, P.ngroups, gtri);
+// Eight threads set winner `ord` up for the tile of row cy, once for all its
+// rows and pixels there.  Each projects and orders the vertices; thread j
+// then takes one attribute (j >> 1: uv with the edge itself, light, normal,
+// position) along one edge (j & 1: to the middle vertex or to the split
+// vertex), as the rasterizer's walk has it: the difference of the ends scaled
+// by 1 / rows, for the half walked upwards with the vertices exchanged.  Thread
+// 0 also takes the mip level, the group and (NRM, F_NORMAL groups) the tangent
+// frame.  NRM = false: draws without normal-mapped groups, whose shade then
+// carries none of that code.
+template <bool NRM>
+__device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev *sg, uint32_t ord, int cy, int j,
+                                             WinnerState &w, WinnerConst &wc) {
+  const int role = j >> 1, k = j & 1;
+  const uint32_t o = ord - 1;
+  const bool tiled = (o >> 31) != 0, up = (o & 1) != 0;
+  const uint32_t gtri = (o >> 1) & 0x3fffffffu;
+  const int g = find_group(sg, P.ngroups, gtri);
   const GroupDev &G = sg[g];
-  int tri = (int)(gtri - G.tri_base);
-  float sx[3], sy[3], sz[3];
-  project_persp(G, tri, P.view, sx, sy, sz);
-  Attr<true> a[3];
-  float z[3], x[3], y[3];
-  int ix[3], iy[3];
+  const int tri = (int)(gtri - G.tri_base);
+  V3 a[3];                       // the thread's attribute, in vertex order below
+  {
+    const float *src = role == 0 ? G.uv : role == 1 ? G.li : role == 2 ? G.vn : G.xyz;
+    const int n = role == 0 ? 2 : 3;
+    src += (size_t)tri * 3 * n;
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    a[k] = a_load<true>(G, tri, k, sz[k]);
-    z[k] = sz[k];
-    x[k] = sx[k]; y[k] = sy[k];
-    ix[k] = f2i(sx[k]); iy[k] = f2i(sy[k]);
+    for (int i = 0; i < 3; i++) a[i] = V3{__ldg(src + i * n), __ldg(src + i * n + 1), role == 0 ? 0.f : __ldg(src + i * n + 2)};
   }
-  const bool mip = (G.flags & F_MIP) != 0;
-  const bool normal = NRM && (G.flags & F_NORMAL) != 0;
-  MipSel ms;
-  ms.fmip = 0; ms.mip = 0; ms.len_mip = 1; ms.len_mip2 = 2; ms.start_mip = 0; ms.start_mip2 = 1;
-  float cx1, cx2, cz1, cz2;
-  Attr<true> c1, c2;
-  if (phase == 0) {
+  float x[3], y[3], z[3];
+  project_persp(G, tri, P.view, x, y, z);
+  int ix[3] = {0, 0, 0}, iy[3] = {0, 0, 0}, v0[3] = {0, 3, 6};   // v0: the vertices' offsets
+  if (!tiled) {
     // direct path: integer vertices (Templates.py:230-231)
-    if (iy[0] > iy[1]) { swap_(iy[0], iy[1]); swap_(ix[0], ix[1]); swap_(z[0], z[1]); swap_(a[0], a[1]); }
-    if (iy[1] > iy[2]) { swap_(iy[1], iy[2]); swap_(ix[1], ix[2]); swap_(z[1], z[2]); swap_(a[1], a[2]); }
-    if (iy[0] > iy[1]) { swap_(iy[0], iy[1]); swap_(ix[0], ix[1]); swap_(z[0], z[1]); swap_(a[0], a[1]); }
-    int x1 = ix[0], x2 = ix[1], x3 = ix[2], y1 = iy[0], y2 = iy[1], y3 = iy[2];
-    float z1 = z[0], z2 = z[1], z3 = z[2];
-    float yd = (float)(y2 - y1) / (float)(y3 - y1);
-    float x4 = (float)x1 + yd * (float)(x3 - x1);
-    float z4 = z1 + yd * (z3 - z1);
-    Attr<true> a4 = a_add(a[0], a_smul(yd, a_sub(a[2], a[0])));
-    if (normal) {
-      if (edge != 1) normal_frame(a, z, st.tan, st.bit);
-      if (!mip) mip_attr_roundtrip<true>(a, z);
-    }
-    if (mip) ms = mip_setup<true>(a, z, true, ix, iy, nullptr, nullptr, G.tex_size, G.mip_bias);
-    float s1, s2, sz1, sz2;
-    Attr<true> sa1, sa2;
-    int n;
-    if (half == 0) {
-      float d = 1.0f / (float)(y2 - y1);
-      s1 = (float)(x2 - x1) * d; s2 = (x4 - (float)x1) * d;
-      sz1 = (z2 - z1) * d; sz2 = (z4 - z1) * d;
-      sa1 = a_mul(a_sub(a[1], a[0]), d); sa2 = a_mul(a_sub(a4, a[0]), d);
-      cx1 = cx2 = (float)x1; cz1 = cz2 = z1; c1 = c2 = a[0];
-      n = cy - y1;
-    } else {
-      float d = 1.0f / (float)(y3 - y2);
-      s1 = (float)(x3 - x2) * d; s2 = ((float)x3 - x4) * d;
-      sz1 = (z3 - z2) * d; sz2 = (z3 - z4) * d;
-      sa1 = a_mul(a_neg(a_sub(a[1], a[2])), d); sa2 = a_mul(a_neg(a_sub(a4, a[2])), d);
-      cx1 = cx2 = (float)x3; cz1 = cz2 = z3; c1 = c2 = a[2];
-      n = y3 - cy;
-    }
-    if (s1 < s2) { swap_(s1, s2); swap_(sz1, sz2); swap_(sa1, sa2); }
-    replay_edges(edge, n, half == 0, cx1, cx2, cz1, cz2, c1, c2, s1, s2, sz1, sz2, sa1, sa2, st);
+#pragma unroll
+    for (int i = 0; i < 3; i++) { ix[i] = f2i(x[i]); iy[i] = f2i(y[i]); }
+  }
+#define SW(i, l) \
+  if (tiled ? y[i] > y[l] : iy[i] > iy[l]) { swap_(x[i], x[l]); swap_(y[i], y[l]); swap_(z[i], z[l]); swap_(ix[i], ix[l]); \
+                                             swap_(iy[i], iy[l]); swap_(a[i], a[l]); swap_(v0[i], v0[l]); }
+  SW(0, 1)
+  SW(1, 2)
+  SW(0, 1)
+#undef SW
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    a[i] = mul3(a[i], z[i]);
+    if (!tiled) x[i] = (float)ix[i];
+  }
+  // heights and x differences: of the integers on the direct path
+  float h21, h32, h31, x21, x32, x31;
+  if (tiled) {
+    h21 = y[1] - y[0]; h32 = y[2] - y[1]; h31 = y[2] - y[0];
+    x21 = x[1] - x[0]; x32 = x[2] - x[1]; x31 = x[2] - x[0];
   } else {
-    // tiled path: float vertices, per-tile restart (Templates.py:93-182)
-    if (y[0] > y[1]) { swap_(y[0], y[1]); swap_(x[0], x[1]); swap_(z[0], z[1]); swap_(a[0], a[1]); }
-    if (y[1] > y[2]) { swap_(y[1], y[2]); swap_(x[1], x[2]); swap_(z[1], z[2]); swap_(a[1], a[2]); }
-    if (y[0] > y[1]) { swap_(y[0], y[1]); swap_(x[0], x[1]); swap_(z[0], z[1]); swap_(a[0], a[1]); }
-    float x1 = x[0], x2 = x[1], x3 = x[2], y1 = y[0], y2 = y[1], y3 = y[2];
-    float z1 = z[0], z2 = z[1], z3 = z[2];
-    float yd = (y2 - y1) / (y3 - y1);
-    float x4 = x1 + yd * (x3 - x1);
-    float z4 = z1 + yd * (z3 - z1);
-    Attr<true> a4 = a_add(a[0], a_smul(yd, a_sub(a[2], a[0])));
+    h21 = (float)(iy[1] - iy[0]); h32 = (float)(iy[2] - iy[1]); h31 = (float)(iy[2] - iy[0]);
+    x21 = (float)(ix[1] - ix[0]); x32 = (float)(ix[2] - ix[1]); x31 = (float)(ix[2] - ix[0]);
+  }
+  const float yd = h21 / h31;
+  const float x4 = x[0] + yd * x31, z4 = z[0] + yd * (z[2] - z[0]);
+  const V3 a4 = add3(a[0], smul3(yd, sub3(a[2], a[0])));
+  const bool mip = (G.flags & F_MIP) != 0, normal = NRM && (G.flags & F_NORMAL) != 0;
+  if (j == 0) {
+    wc.g = g;
+    wc.fmip = 0.f;
+    wc.mip = 0;
+    Attr<false> uv[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) uv[i].uv = V2{a[i].x, a[i].y};
     if (normal) {
-      if (edge != 1) normal_frame(a, z, st.tan, st.bit);
-      if (!mip) mip_attr_roundtrip<true>(a, z);
+      const float *xyz = G.xyz + (size_t)tri * 9;
+      V3 p[3] = {mul3(ld3(xyz + v0[0]), z[0]), mul3(ld3(xyz + v0[1]), z[1]), mul3(ld3(xyz + v0[2]), z[2])};
+      normal_frame(uv, p, z, wc.tan, wc.bit);
     }
     if (mip) {
-      if (P.mipc) {
-        mip_attr_roundtrip<true>(a, z);
-        float2 mc = P.mipc[gtri];
-        ms.fmip = mc.x; ms.mip = (int)mc.y;
-      } else {
-        ms = mip_setup<true>(a, z, false, nullptr, nullptr, x, y, G.tex_size, G.mip_bias);
-      }
-    }
-    int tileY = cy / TILE;
-    float yMin = (float)tileY * 16.f, yMax = ((float)tileY + 1.f) * 16.f - 1.f;
-    float s1, s2, sz1, sz2;
-    Attr<true> sa1, sa2;
-    if (half == 0) {
-      float d = 1.0f / (y2 - y1);
-      s1 = (x2 - x1) * d; s2 = (x4 - x1) * d;
-      sz1 = (z2 - z1) * d; sz2 = (z4 - z1) * d;
-      sa1 = a_mul(a_sub(a[1], a[0]), d); sa2 = a_mul(a_sub(a4, a[0]), d);
-      if (s1 < s2) { swap_(s1, s2); swap_(sz1, sz2); swap_(sa1, sa2); }
-      int cy0 = f2i(clampf_(y1, yMin, yMax));
-      float dy = (float)cy0 - y1;
-      cx1 = x1 + dy * s1; cx2 = x1 + dy * s2; cz1 = z1 + dy * sz1; cz2 = z1 + dy * sz2;
-      c1 = a_add(a[0], a_smul(dy, sa1)); c2 = a_add(a[0], a_smul(dy, sa2));
-      replay_edges(edge, cy - cy0, true, cx1, cx2, cz1, cz2, c1, c2, s1, s2, sz1, sz2, sa1, sa2, st);
-    } else {
-      float d = 1.0f / (y3 - y2);
-      s1 = (x3 - x2) * d; s2 = (x3 - x4) * d;
-      sz1 = (z3 - z2) * d; sz2 = (z3 - z4) * d;
-      sa1 = a_mul(a_neg(a_sub(a[1], a[2])), d); sa2 = a_mul(a_neg(a_sub(a4, a[2])), d);
-      if (s1 < s2) { swap_(s1, s2); swap_(sz1, sz2); swap_(sa1, sa2); }
-      int cy0 = f2i(clampf_(y3, yMin, yMax));
-      float dy = (float)cy0 - y3;
-      cx1 = x3 + dy * s1; cx2 = x3 + dy * s2; cz1 = z3 + dy * sz1; cz2 = z3 + dy * sz2;
-      c1 = a_add(a[2], a_smul(dy, sa1)); c2 = a_add(a[2], a_smul(dy, sa2));
-      replay_edges(edge, cy0 - cy, false, cx1, cx2, cz1, cz2, c1, c2, s1, s2, sz1, sz2, sa1, sa2, st);
+      MipSel ms = mip_setup<false>(uv, z, !tiled, ix, iy, x, y, G.tex_size, G.mip_bias);
+      wc.fmip = ms.fmip;
+      wc.mip = ms.mip;
     }
   }
-  if (edge != 1) { st.fmip = ms.fmip; st.mip = ms.mip; st.g = g; }
+  if ((mip || normal) && (role == 0 || role == 3)) {   // the round trip of uv and position (mip_setup)
+#pragma unroll
+    for (int i = 0; i < 3; i++) a[i] = mul3(div3(a[i], z[i]), z[i]);
+  }
+  // the half's first vertex, its slopes to the middle and to the split vertex
+  const float d = 1.0f / (up ? h32 : h21);
+  const float xs = up ? x[2] : x[0], ys = up ? y[2] : y[0], zs = up ? z[2] : z[0];
+  const float s1 = (up ? x32 : x21) * d, s2 = (up ? x[2] - x4 : x4 - x[0]) * d;
+  const float sz = (k ? (up ? z[2] - z4 : z4 - z[0]) : (up ? z[2] - z[1] : z[1] - z[0])) * d, s = k ? s2 : s1;
+  const V3 from = up ? a[2] : a[0];
+  V3 sa = sub3(k ? a4 : a[1], from);
+  sa = mul3(up ? neg3(sa) : sa, d);
+  const float yMin = (float)(cy / TILE) * 16.f;
+  const int cy0 = tiled ? f2i(clampf_(ys, yMin, yMin + 15.f)) : (up ? iy[2] : iy[0]);
+  const float dy = (float)cy0 - ys;          // tiled path: restarted at the tile's first row
+  const int e = (s1 < s2) ? 1 - k : k;       // the larger slope is the first chain's
+  float *st = reinterpret_cast<float *>(&w.start[e]), *sp = reinterpret_cast<float *>(&w.step[e]);
+  const V3 c = tiled ? add3(from, smul3(dy, sa)) : from;
+  if (up) sa = neg3(sa);
+  if (role == 0) {
+    st[0] = tiled ? xs + dy * s : xs;
+    st[1] = tiled ? zs + dy * sz : zs;
+    sp[0] = up ? -s : s;
+    sp[1] = up ? -sz : sz;
+    if (k == 0) w.y0 = cy0;
+    st[2] = c.x; st[3] = c.y;
+    sp[2] = sa.x; sp[3] = sa.y;
+  } else {
+    st += 1 + 3 * role; sp += 1 + 3 * role;
+    st[0] = c.x; st[1] = c.y; st[2] = c.z;
+    sp[0] = sa.x; sp[1] = sa.y; sp[2] = sa.z;
+  }
 }
 
-__device__ __forceinline__ void shade_row(const DrawParams &P, const GroupDev *sg, uint32_t ord, int cy, RowState &st) {
-  shade_row_edge(P, sg, ord, cy, 2, st);
+// The chain e of winner w on row cy: the rasterizer's additions.
+__device__ __forceinline__ void replay_edge(const WinnerState &w, int e, int cy, EdgeState &out) {
+  EdgeState c = w.start[e];
+  const EdgeState s = w.step[e];
+  for (int r = iabs_(cy - w.y0); r > 0; r--) {
+    c.cx += s.cx; c.cz += s.cz;
+    c.c = a_add(c.c, s.c);
+  }
+  out = c;
 }
 
 // av_draw_multi.c:30-105: the 4-way terrain blend of a F_MULTI group.  Its
@@ -1739,16 +1702,17 @@ __device__ __forceinline__ void shade_row(const DrawParams &P, const GroupDev *s
 __device__ __forceinline__ void shade_multi(const DrawParams &P, const GroupDev *G, size_t pix, float t, float tz,
                                             V2 uvi, const RowState &st) {
   float omt = 1 - t;
+  const Attr<true> &c1 = st.e[0].c, &c2 = st.e[1].c;
   Taps q = make_taps(uvi, tz, G[0].tex_size, 0);
   V3 tx[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) tx[k] = bilerp_rgb(q, G[k].tex);
-  V3 col = mul3(add3(smul3(omt, st.c2.li), smul3(t, st.c1.li)), tz);
-  V3 nrm = fast_normalize(mul3(add3(smul3(omt, st.c2.n), smul3(t, st.c1.n)), tz));
+  V3 col = mul3(add3(smul3(omt, c2.li), smul3(t, c1.li)), tz);
+  V3 nrm = fast_normalize(mul3(add3(smul3(omt, c2.n), smul3(t, c1.n)), tz));
   V3 ldir{P.light.ldir[0], P.light.ldir[1], P.light.ldir[2]};
   V3 lint{P.light.lint[0], P.light.lint[1], P.light.lint[2]};
   V3 dc = smul3(fmaxf(0.f, dot3(nrm, ldir)), lint);
-  V3 cpos = mul3(add3(smul3(omt, st.c2.p), smul3(t, st.c1.p)), tz);
+  V3 cpos = mul3(add3(smul3(omt, c2.p), smul3(t, c1.p)), tz);
   float m = (cpos.y - 15.f) / 4.f;
   m = fminf(fmaxf(m, 0.f), 1.f);
   float ny = fmaxf(0.f, fabsf(nrm.y) - 0.33f) * 1.5f;
@@ -1823,8 +1787,9 @@ __device__ __forceinline__ V3 bilerp_nm(const Taps &q, const uchar4 *__restrict_
 // av_draw_normmap_mip.c:73-160.  The light comes from the draw's first
 // cascade (sample_shadow5), 1 without one.  Kept out of line so that the
 // other materials keep their registers.
-__device__ __noinline__ void shade_normal(const DrawParams &P, const GroupDev &G, size_t pix, float t, float tz,
-                                          V2 uvi, const RowState &st, MipSel ms) {
+__device__ __forceinline__ void shade_normal(const DrawParams &P, const GroupDev &G, size_t pix, float t, float tz,
+                                          V2 uvi, const RowState &st, const WinnerConst &wc, MipSel ms) {
+  const Attr<true> &c1 = st.e[0].c, &c2 = st.e[1].c;
   const bool mip = (G.flags & F_MIP) != 0;
   float omt = 1 - t;
   Taps q = make_taps(uvi, tz, mip ? ms.len_mip : G.tex_size, mip ? ms.start_mip : 0);
@@ -1834,16 +1799,16 @@ __device__ __noinline__ void shade_normal(const DrawParams &P, const GroupDev &G
   if (mip) {
     Taps q2 = make_taps(uvi, tz, ms.len_mip2, ms.start_mip2);
     float ofm = 1 - ms.fmip;
-    V3 c2 = bilerp_rgb(q2, G.tex);
-    outR = ofm * outR + ms.fmip * c2.x;
-    outG = ofm * outG + ms.fmip * c2.y;
-    outB = ofm * outB + ms.fmip * c2.z;
+    V3 cb = bilerp_rgb(q2, G.tex);
+    outR = ofm * outR + ms.fmip * cb.x;
+    outG = ofm * outG + ms.fmip * cb.y;
+    outB = ofm * outB + ms.fmip * cb.z;
     tg = add3(smul3(ofm, tg), smul3(ms.fmip, bilerp_nm(q2, G.nm)));
   }
   float light = 1;
   if (P.nsh > 0) {
     const ShadowDev &sh = P.sh[0];
-    V3 pos = sub3(mul3(add3(smul3(omt, st.c2.p), smul3(t, st.c1.p)), tz), V3{sh.pos[0], sh.pos[1], sh.pos[2]});
+    V3 pos = sub3(mul3(add3(smul3(omt, c2.p), smul3(t, c1.p)), tz), V3{sh.pos[0], sh.pos[1], sh.pos[2]});
     float depth = dot3(pos, V3{sh.vv[0], sh.vv[1], sh.vv[2]});
     float wS = (float)(sh.dim / 2);
     float sfx = (dot3(pos, V3{sh.vv[3], sh.vv[4], sh.vv[5]}) * sh.scale) + wS;
@@ -1852,15 +1817,15 @@ __device__ __noinline__ void shade_normal(const DrawParams &P, const GroupDev &G
   } else {
     light = 1 - 0.f;
   }
-  V3 col = mul3(add3(smul3(omt, st.c2.li), smul3(t, st.c1.li)), tz);
-  V3 norm = fast_normalize(mul3(add3(smul3(omt, st.c2.n), smul3(t, st.c1.n)), tz));
+  V3 col = mul3(add3(smul3(omt, c2.li), smul3(t, c1.li)), tz);
+  V3 norm = fast_normalize(mul3(add3(smul3(omt, c2.n), smul3(t, c1.n)), tz));
   tg = sub3(mul3(div3(tg, 255.f), 2.f), V3{1.f, 1.f, 1.f});
   tg = fast_normalize(tg);
-  norm = fast_normalize(add3(add3(smul3(tg.z, norm), smul3(-tg.y, st.tan)), smul3(-tg.x, st.bit)));
+  norm = fast_normalize(add3(add3(smul3(tg.z, norm), smul3(-tg.y, wc.tan)), smul3(-tg.x, wc.bit)));
   V3 vp{P.view.pos[0], P.view.pos[1], P.view.pos[2]};
   V3 lint{P.light.lint[0], P.light.lint[1], P.light.lint[2]};
   V3 ldir{P.light.ldir[0], P.light.ldir[1], P.light.ldir[2]};
-  V3 pos = mul3(add3(smul3(omt, st.c2.p), smul3(t, st.c1.p)), tz);
+  V3 pos = mul3(add3(smul3(omt, c2.p), smul3(t, c1.p)), tz);
   V3 spec;
   if (mip) {
     V3 a = sub3(pos, vp);
@@ -1903,16 +1868,16 @@ __device__ __noinline__ void shade_normal(const DrawParams &P, const GroupDev &G
 // Shades pixel ax of row cy from its winner's row state.
 template <bool NRM = true>
 __device__ __forceinline__ void shade_from_row(const DrawParams &P, const GroupDev *sg, int ax, int cy,
-                                               const RowState &st) {
-  const GroupDev &G = sg[st.g];
+                                               const RowState &st, const WinnerConst &wc) {
+  const GroupDev &G = sg[wc.g];
   const bool mip = (G.flags & F_MIP) != 0;
   MipSel ms;
-  ms.fmip = st.fmip; ms.mip = st.mip;
+  ms.fmip = wc.fmip; ms.mip = wc.mip;
   ms.len_mip = 1 << ms.mip; ms.len_mip2 = ms.len_mip << 1;
   ms.start_mip = ((1 << (2 * ms.mip)) - 1) / 3;            // sum of 4^i for i < mip
   ms.start_mip2 = ms.start_mip + ms.len_mip * ms.len_mip;
-  const float cx1 = st.cx1, cx2 = st.cx2, cz1 = st.cz1, cz2 = st.cz2;
-  const Attr<true> c1 = st.c1, c2 = st.c2;
+  const float cx1 = st.e[0].cx, cx2 = st.e[1].cx, cz1 = st.e[0].cz, cz2 = st.e[1].cz;
+  const Attr<true> &c1 = st.e[0].c, &c2 = st.e[1].c;
   float t = ((float)ax - cx2) / (cx1 - cx2);
   t = clamp_t(t);
   float tz = 1.0f / ((1 - t) * cz2 + t * cz1);
@@ -1923,7 +1888,7 @@ __device__ __forceinline__ void shade_from_row(const DrawParams &P, const GroupD
     return;
   }
   if (NRM && (G.flags & F_NORMAL)) {
-    shade_normal(P, G, (size_t)P.view.w * cy + ax, t, tz, uvi, st, ms);
+    shade_normal(P, G, (size_t)P.view.w * cy + ax, t, tz, uvi, st, wc, ms);
     return;
   }
   float outR, outG, outB;
@@ -1961,78 +1926,88 @@ __device__ __forceinline__ void shade_from_row(const DrawParams &P, const GroupD
   P.db[pix] = tz;
 }
 
-// Replays the winning fragment of pixel (ax, cy) and shades it.
-__device__ __forceinline__ void shade_pixel(const DrawParams &P, const GroupDev *sg, int ax, int cy, uint64_t key) {
-  uint32_t ord = 0xffffffffu - (uint32_t)key;
-  if (ord == 0) return;
-  RowState st;
-  shade_row(P, sg, ord, cy, st);
-  shade_from_row(P, sg, ax, cy, st);
-}
-
 // Shared memory of shade_tile for a block of NT threads (16 x NT/16 pixels).
+constexpr int WINNERS = 32;        // winners set up at a time
 template <int NT>
 struct ShadeSmem {
-  unsigned long long hkey[NT];   // open-addressing table of (winner, row) keys
-  int hent[NT];                  // its entry numbers
-  unsigned long long ekey[NT];   // entry -> key
-  int nent;
-  RowState rs[NT];
+  uint32_t hkey[NT];               // open-addressing table of the tile's winners (order keys)
+  uint16_t hent[NT];               // its entry numbers
+  uint32_t ekey[NT];               // entry -> order key
+  int nent, npair;
+  uint16_t pair[NT];               // (winner, row) pairs: table slot << 4 | row
+  WinnerConst wc[WINNERS];
+  WinnerState ws[WINNERS];
+  RowState rs[NT];                 // their edge chains, indexed alike
 };
 
-// Shades the 16 x (NT/16) pixels at (x0, y0): the block finds the distinct
-// (winner, row) pairs among its pixels (a bounded open-addressing table in
-// shared memory), two threads per pair set up the triangle and replay its
-// row (one edge chain each), then every pixel shades from its pair's row
-// state.  The arithmetic is shade_pixel's, done once per pair instead of once
-// per pixel.
+// Shades the 16 x (NT/16) pixels at (x0, y0) in three steps.  The block finds
+// the distinct winners (triangle halves) among its pixels, through a bounded
+// open-addressing table in shared memory, and their (winner, row) pairs;
+// eight threads a winner set it up for the tile; two threads a pair replay its
+// edge chains; then every pixel shades from its pair.  The arithmetic is the
+// rasterizer's walk, the set-up done once a winner, the additions once a pair.
+//
+// A tile of the 1080p / 1.04M-triangle frame has 5.5 winners and 41 pairs (of
+// 256 pixels).  With every pair set up by itself (projection, mip level, slopes:
+// most of the kernel's instructions, on three of the block's eight warps) the
+// kernel took 177 us of that frame and 95M warp instructions; set up by winner
+// 149 us, with the pairs of the whole block replayed together 142 us and 71M,
+// with eight threads a winner instead of two 137 us.  What is left is waiting at
+// the barriers between the steps (6.9 of 14 cycles an instruction) with four
+// blocks of 64 registers an SM.  8-row tiles (half the threads a block) take 12%
+// longer; two or three blocks an SM 3-10%.
 template <int NT, bool NRM = true>
 __device__ __forceinline__ void shade_tile(const DrawParams &P, const GroupDev *sg, int x0, int y0, ShadeSmem<NT> &sm) {
-  const unsigned long long EMPTY = ~0ull;
-  int tid = threadIdx.x;
-  int ax = x0 + (tid & 15), cy = y0 + (tid >> 4);
-  bool in = ax < P.view.w && cy < P.view.h;
-  uint32_t ord = in ? 0xffffffffu - (uint32_t)P.keys[(size_t)P.view.w * cy + ax] : 0u;
-  bool valid = ord != 0;
-  sm.hkey[tid] = EMPTY;
-  if (tid == 0) sm.nent = 0;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int ax = x0 + (tid & 15), cy = y0 + (tid >> 4);
+  const bool in = ax < P.view.w && cy < P.view.h;
+  const uint32_t ord = in ? 0xffffffffu - (uint32_t)P.keys[(size_t)P.view.w * cy + ax] : 0u;
+  sm.hkey[tid] = 0u;                     // 0: no winner has order 0
+  if (tid == 0) sm.nent = sm.npair = 0;
   __syncthreads();
+  // a row of the tile lies in one warp, so the first lane of each (winner,
+  // row) is the pair's only one in the block
+  const unsigned row = __match_any_sync(FULL, ord) & (lane < 16 ? 0xffffu : 0xffff0000u);
+  const int leader = __ffs(row) - 1;
+  const bool leads = ord != 0 && lane == leader;
   int slot = 0;
-  // the lanes of a warp with the same (winner, row) -- often a whole row of
-  // the tile -- insert it once, through their first lane
-  unsigned long long k = valid ? (((unsigned long long)ord << 32) | (uint32_t)cy) : EMPTY;
-  const unsigned peers = __match_any_sync(FULL, k);
-  const int leader = __ffs(peers) - 1;
-  if (valid && (tid & 31) == leader) {
-    uint32_t h = ((ord * 2654435761u) ^ ((uint32_t)cy * 40503u)) % NT;
+  if (leads) {
+    uint32_t h = (ord * 2654435761u >> 16) % NT;
     for (int i = 0; i < NT; i++) {       // at most NT keys: always finds a slot
-      unsigned long long prev = atomicCAS(&sm.hkey[h], EMPTY, k);
-      if (prev == EMPTY) {
+      uint32_t prev = atomicCAS(&sm.hkey[h], 0u, ord);
+      if (prev == 0u) {
         int e = atomicAdd(&sm.nent, 1);
-        sm.hent[h] = e;
-        sm.ekey[e] = k;
-        slot = (int)h;
-        break;
+        sm.hent[h] = (uint16_t)e;
+        sm.ekey[e] = ord;
       }
-      if (prev == k) {
-        slot = (int)h;
-        break;
-      }
+      if (prev == 0u || prev == ord) { slot = (int)h; break; }
       h = (h + 1) % NT;
     }
   }
-  slot = __shfl_sync(FULL, slot, leader);
+  const unsigned leaders = __ballot_sync(FULL, leads);
+  int first = 0;
+  if (lane == 0) first = atomicAdd(&sm.npair, __popc(leaders));
+  const int pair = __shfl_sync(FULL, first, 0) + __popc(leaders & ((1u << leader) - 1u));   // of this lane's pixel
+  if (leads) sm.pair[pair] = (uint16_t)(slot << 4 | tid >> 4);
   __syncthreads();
-  int ne = sm.nent;
-  for (int j = tid; j < 2 * ne; j += NT) {   // two threads a pair, one edge chain each
-    unsigned long long k = sm.ekey[j >> 1];
-    shade_row_edge<NRM>(P, sg, (uint32_t)(k >> 32), (int)(uint32_t)k, j & 1, sm.rs[j >> 1]);
+  const int nw = sm.nent, npairs = sm.npair;
+  for (int base = 0; base < nw; base += WINNERS) {
+    const int m = min(WINNERS, nw - base);
+    for (int j = tid; j < 8 * m; j += NT)
+      winner_setup<NRM>(P, sg, sm.ekey[base + (j >> 3)], y0, j & 7, sm.ws[j >> 3], sm.wc[j >> 3]);
+    __syncthreads();
+    for (int j = tid; j < 2 * npairs; j += NT) {
+      const int info = sm.pair[j >> 1], w = (int)sm.hent[info >> 4] - base;
+      if ((unsigned)w < (unsigned)m) replay_edge(sm.ws[w], j & 1, y0 + (info & 15), sm.rs[j >> 1].e[j & 1]);
+    }
+    __syncthreads();
+    if (ord != 0) {
+      const int w = (int)sm.hent[sm.pair[pair] >> 4] - base;
+      if ((unsigned)w < (unsigned)m) shade_from_row<NRM>(P, sg, ax, cy, sm.rs[pair], sm.wc[w]);
+    }
+    __syncthreads();                     // the next winners (or the next tile) reuse the shared memory
   }
-  __syncthreads();
-  if (valid) shade_from_row<NRM>(P, sg, ax, cy, sm.rs[sm.hent[slot]]);
-  __syncthreads();                       // the next tile reuses the shared memory
 }
-
 
 // one 256-thread block per 16x16 tile
 // NRM: the draw has normal-mapped groups
