@@ -167,7 +167,8 @@ struct axr_ctx {
   cudaEvent_t ev_lights = nullptr;
   bool lights_used = false;
   uint16_t *post[3] = {nullptr, nullptr, nullptr};   // dof's gather target (SSRO/SSGO/SSBO)
-  uint16_t *bloom = nullptr;                           // the bloom's 9 half-resolution planes
+  uint16_t *bloom = nullptr;                           // the bloom's 3 half-resolution planes
+  int ssao_blocks = 4;                       // resident 256-thread blocks of k_ssao per SM
   int light_blocks = 4;                      // resident 256-thread blocks of k_vert_light per SM
   // launch accounting and optional per-kernel CUDA-event timing
   int64_t launches = 0;
@@ -578,6 +579,8 @@ int axr_create(int w, int h, int device, axr_ctx **out) {
   }
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->light_blocks, k_vert_light, 256, 0);
   if (c->light_blocks < 1) c->light_blocks = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->ssao_blocks, k_ssao, 256, 0);
+  if (c->ssao_blocks < 1) c->ssao_blocks = 1;
   // initial tile-unit queue (grows after an overflow); AXR_UNIT_QUEUE overrides
   uint32_t units0 = 1u << 22;
   if (const char *e = getenv("AXR_UNIT_QUEUE")) {
@@ -1132,7 +1135,7 @@ int axr_read_frame_rgb8_async(axr_ctx *c, float exposure, uint8_t *rgb, int64_t 
   }
   cudaStream_t s = c->stream;
   launch(c, s, "k_pack_rgb8", [&] {
-    k_pack_rgb8<<<grid_for(c, (long)n, 256, 8), 256, 0, s>>>(c->ro, c->go, c->bo, (int)n, exposure, sl.stage);
+    k_pack_rgb8<<<grid_for(c, (long)n / 4, 256, 8), 256, 0, s>>>(c->ro, c->go, c->bo, (int)n, exposure, sl.stage);
   });
   CK(cudaGetLastError());
   CK(cudaEventRecord(sl.staged, s));
@@ -1205,7 +1208,7 @@ int axr_gamma(axr_ctx *c, float ex) {
   int rc = check_ctx(c);
   if (rc) return rc;
   long n = (long)c->w * c->h;
-  launch(c, c->stream, "k_gamma", [&] { k_gamma<<<grid_for(c, n, 256, 8), 256, 0, c->stream>>>(c->ro, c->go, c->bo, (int)n, ex); });
+  launch(c, c->stream, "k_gamma", [&] { k_gamma<<<grid_for(c, n / 8, 256, 8), 256, 0, c->stream>>>(c->ro, c->go, c->bo, (int)n, ex); });
   CK(cudaGetLastError());
   return 0;
 }
@@ -1218,7 +1221,7 @@ int axr_ssao(axr_ctx *c, const float *rnd, int n) {
   SsaoParams S;
   memcpy(S.rnd, rnd, sizeof S.rnd);
   S.sscale = c->sscale;
-  dim3 grid(c->w / 16, c->h / 16);
+  const int grid = std::min((c->w / 16) * (c->h / 16), c->sms * c->ssao_blocks);
   launch(c, c->stream, "k_ssao", [&] { k_ssao<<<grid, 256, 0, c->stream>>>(c->ro, c->go, c->bo, c->db, c->w, c->h, S); });
   CK(cudaGetLastError());
   return 0;
@@ -1237,9 +1240,12 @@ int axr_dof(axr_ctx *c, float focus) {
                                        c->post[2]);
   });
   // Ops.py:993-995 copies the gather back; rows below the covered region keep their colour
-  size_t bytes = (size_t)c->w * (c->h / 16 * 16) * 2;
-  uint16_t *dst[3] = {c->ro, c->go, c->bo};
-  for (int k = 0; k < 3; k++) CK(cudaMemcpyAsync(dst[k], c->post[k], bytes, cudaMemcpyDeviceToDevice, c->stream));
+  int n8 = c->w * (c->h / 16 * 16) / 8;
+  uint4 *const *f = reinterpret_cast<uint4 *const *>(c->post);
+  launch(c, c->stream, "k_copy3", [&] {
+    k_copy3<<<grid_for(c, n8, 256, 8), 256, 0, c->stream>>>(reinterpret_cast<uint4 *>(c->ro), reinterpret_cast<uint4 *>(c->go),
+                                                              reinterpret_cast<uint4 *>(c->bo), f[0], f[1], f[2], n8);
+  });
   CK(cudaGetLastError());
   return 0;
 }
@@ -1249,26 +1255,16 @@ int axr_bloom(axr_ctx *c) {
   if (rc) return rc;
   int wf = c->w / 2, hf = c->h / 2;
   if (hf < 3) return 0;                              // no row of the bright pass
-  size_t plane = (size_t)wf * (hf + 8);
-  if (!c->bloom) {
-    if (cudaMalloc(&c->bloom, plane * 9 * 2) != cudaSuccess) return fail(AXR_ENOMEM, "bloom planes");
-    CK(cudaMemsetAsync(c->bloom, 0, plane * 9 * 2, c->stream));   // rows no pass writes read 0
-  }
+  size_t plane = (size_t)wf * (hf - 1);
+  if (!c->bloom && cudaMalloc(&c->bloom, plane * 3 * 2) != cudaSuccess) return fail(AXR_ENOMEM, "bloom planes");
   BloomPlanes B;
-  for (int k = 0; k < 3; k++) {
-    B.br[k] = c->bloom + plane * k;
-    B.hb[k] = c->bloom + plane * (3 + k);
-    B.vb[k] = c->bloom + plane * (6 + k);
-  }
-  int bx = (wf + 127) / 128;
-  launch(c, c->stream, "k_bloom_bright", [&] {
-    k_bloom_bright<<<dim3(bx, hf - 2), 128, 0, c->stream>>>(c->ro, c->go, c->bo, wf, hf, B);
+  for (int k = 0; k < 3; k++) B.hb[k] = c->bloom + plane * k;
+  launch(c, c->stream, "k_bloom_h", [&] {
+    k_bloom_h<<<dim3((wf + BLOOM_W - 1) / BLOOM_W, hf - 1), BLOOM_W, 0, c->stream>>>(c->ro, c->go, c->bo, wf, hf, B);
   });
-  launch(c, c->stream, "k_bloom_blur_h", [&] { k_bloom_blur<true><<<dim3(bx, hf - 1), 128, 0, c->stream>>>(wf, hf, B); });
-  launch(c, c->stream, "k_bloom_blur_v", [&] { k_bloom_blur<false><<<dim3(bx, hf - 1), 128, 0, c->stream>>>(wf, hf, B); });
-  int fx = (2 * wf + 127) / 128;
-  launch(c, c->stream, "k_bloom_add", [&] {
-    k_bloom_add<<<dim3(fx, 2 * hf), 128, 0, c->stream>>>(c->ro, c->go, c->bo, c->w, wf, hf, B);
+  launch(c, c->stream, "k_bloom_v", [&] {
+    k_bloom_v<<<dim3((wf + BLOOM_TW - 1) / BLOOM_TW, (hf + BLOOM_TH - 1) / BLOOM_TH, 3), BLOOM_V_THREADS, 0, c->stream>>>(
+        c->ro, c->go, c->bo, c->w, wf, hf, B);
   });
   CK(cudaGetLastError());
   return 0;
