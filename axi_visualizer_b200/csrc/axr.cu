@@ -766,15 +766,18 @@ int axr_vert_light(axr_ctx *c, const uint8_t *mask, int ngroups, const float *di
   L.dint = d + off[0]; L.ddir = d + off[1]; L.pint = d + off[2]; L.ppos = d + off[3];
   L.sint = d + off[4]; L.sdir = d + off[5]; L.spos = d + off[6];
   L.nd = ndirs; L.np = npoints; L.ns = nspots; L.amb = amb;
+  VertJobs J;
+  int nj = 0, most = 0;
   for (int g = 0; g < ngroups; g++) {
-    if (mask && !mask[g]) continue;
     const Group &G = c->groups[g];
-    int nv = G.ntris * 3;
-    if (!nv) continue;
-    launch(c, c->stream, "k_vert_light", [&] {
-      k_vert_light<<<grid_for(c, nv, 256, c->light_blocks), 256, 0, c->stream>>>(G.xyz, G.vn, G.li, nv, L);
-    });
+    if ((mask && !mask[g]) || !G.ntris) continue;
+    J.g[nj++] = {G.xyz, G.vn, G.li, G.ntris * 3};
+    most = std::max(most, G.ntris * 3);
   }
+  if (nj)
+    launch(c, c->stream, "k_vert_light", [&] {
+      k_vert_light<<<dim3(grid_for(c, most / 4 + 1, 256, c->light_blocks), nj), 256, 0, c->stream>>>(J, L);
+    });
   CK(cudaGetLastError());
   c->amb = amb;
   return 0;
