@@ -754,15 +754,12 @@ __device__ __forceinline__ void block_items(uint32_t *items, uint32_t cap_items,
   for (int i = threadIdx.x; i < 2 * LEN_BUCKETS; i += blockDim.x) hist[i / LEN_BUCKETS][i % LEN_BUCKETS] = 0;
   __syncthreads();
   const int k = alpha ? 1 : 0;
-  uint32_t rk[MAX_CHUNKS];
-#pragma unroll
-  for (int c = 0; c < MAX_CHUNKS; c++) {
-    rk[c] = 0;
-    if (c < nch) {
-      int len = min(cl, rows - c * cl);
-      rk[c] = atomicAdd(&hist[k][LEN_BUCKETS - 1 - min(len, LEN_BUCKETS - 1)], 1u);   // bucket 0: the longest
-    }
-  }
+  // its chunks are cl rows long but for the last: bucket 0 holds the longest
+  const int bf = LEN_BUCKETS - 1 - min(cl, LEN_BUCKETS - 1);
+  const int bl = LEN_BUCKETS - 1 - min(rows - (nch - 1) * cl, LEN_BUCKETS - 1);
+  uint32_t rf = 0, rl = 0;
+  if (nch > 1) rf = atomicAdd(&hist[k][bf], (uint32_t)(nch - 1));
+  if (nch > 0) rl = atomicAdd(&hist[k][bl], 1u);
   __syncthreads();
   if (threadIdx.x < 2) {
     uint32_t run = 0;
@@ -774,15 +771,11 @@ __device__ __forceinline__ void block_items(uint32_t *items, uint32_t cap_items,
     bbase[threadIdx.x] = run ? atomicAdd(&ctr[threadIdx.x ? ctr_a : ctr_o], run) : 0u;
   }
   __syncthreads();
-#pragma unroll
-  for (int c = 0; c < MAX_CHUNKS; c++) {
-    if (c < nch) {
-      int len = min(cl, rows - c * cl);
-      uint32_t p = bbase[k] + hist[k][LEN_BUCKETS - 1 - min(len, LEN_BUCKETS - 1)] + rk[c];
-      uint32_t item = (pos << CHUNK_BITS) | (uint32_t)c;
-      if (!alpha) items[p] = item;
-      else items[cap_items - 1 - p] = item;
-    }
+  for (int c = 0; c < nch; c++) {
+    uint32_t p = bbase[k] + (c < nch - 1 ? hist[k][bf] + rf + c : hist[k][bl] + rl);
+    uint32_t item = (pos << CHUNK_BITS) | (uint32_t)c;
+    if (!alpha) items[p] = item;
+    else items[cap_items - 1 - p] = item;
   }
   __syncthreads();   // the next call reuses hist and bbase
 }
@@ -1282,66 +1275,91 @@ __global__ void __launch_bounds__(128, ALPHA ? 6 : 8) k_raster_small(DrawParams 
 
 // ------------------------------------------------------------ coarse binning
 
-// coarse.c:17-125 in tile units; calls emit(tile) for every bin entry
-template <class F>
-__device__ __forceinline__ void coarse_walk(const float sx[3], const float sy[3], int wc, int hc, F emit) {
-  float x1 = sx[0] / 16.f - 0.5f, x2 = sx[1] / 16.f - 0.5f, x3 = sx[2] / 16.f - 0.5f;
-  float y1 = sy[0] / 16.f - 0.5f, y2 = sy[1] / 16.f - 0.5f, y3 = sy[2] / 16.f - 0.5f;
-  float t;
-  if (y1 > y2) { t = y1; y1 = y2; y2 = t; t = x1; x1 = x2; x2 = t; }
-  if (y2 > y3) { t = y2; y2 = y3; y3 = t; t = x2; x2 = x3; x3 = t; }
-  if (y1 > y2) { t = y1; y1 = y2; y2 = t; t = x1; x1 = x2; x2 = t; }
-  float x4 = (x1 + ((y2 - y1) / (y3 - y1)) * (x3 - x1));
-  float y4 = y2;
-  float s1 = (x2 - x1) / (y2 - y1);
-  float s2 = (x4 - x1) / (y4 - y1);
-  float cx1 = x1, cx2 = x1;
-  if (s1 < s2) { t = s1; s1 = s2; s2 = t; }
-  float sbias = 1.f + floorf(y1) - y1;
-  float wcm1 = (float)wc - 1;
-  int guard = 0;
-  if (y1 != y2) {
-    for (int cy = f2i(floorf(y1)); (float)cy <= ceilf(y2) && guard < LOOP_LIMIT; cy++, guard++) {
-      float mx1 = cx1 + sbias * s1;
-      if (s1 < 0) mx1 -= s1;
-      float mx2 = cx2 + sbias * s2;
-      if (s2 > 0) mx2 -= s2;
-      mx1 = fminf(mx1, wcm1);
-      mx2 = fmaxf(mx2, 0.f);
-      if (cy >= 0 && cy < hc) {
-        int a1 = f2i(floorf(mx2));
-        float hb = ceilf(mx1);
-        for (int ax = a1; (float)ax <= hb && ax < wc; ax++) emit(wc * cy + ax);
-      }
-      cx1 += s1;
-      cx2 += s2;
+// coarse.c:17-125 in tile units, one tile row at a time: the bottom half's
+// rows upwards, then the top half's downwards.
+struct CoarseWalk {
+  float x2, x3, y2, y3, x4, wcm1;
+  float s1, s2, cx1, cx2, sbias, bound;
+  int cy, half, guard, wc, hc;
+
+  __device__ __forceinline__ void init(const float sx[3], const float sy[3], int wc_, int hc_) {
+    float x1 = sx[0] / 16.f - 0.5f, y1 = sy[0] / 16.f - 0.5f;
+    x2 = sx[1] / 16.f - 0.5f; x3 = sx[2] / 16.f - 0.5f;
+    y2 = sy[1] / 16.f - 0.5f; y3 = sy[2] / 16.f - 0.5f;
+    if (y1 > y2) { swap_(y1, y2); swap_(x1, x2); }
+    if (y2 > y3) { swap_(y2, y3); swap_(x2, x3); }
+    if (y1 > y2) { swap_(y1, y2); swap_(x1, x2); }
+    x4 = (x1 + ((y2 - y1) / (y3 - y1)) * (x3 - x1));
+    s1 = (x2 - x1) / (y2 - y1);
+    s2 = (x4 - x1) / (y2 - y1);
+    cx1 = x1; cx2 = x1;
+    if (s1 < s2) swap_(s1, s2);
+    sbias = 1.f + floorf(y1) - y1;
+    wc = wc_; hc = hc_; wcm1 = (float)wc - 1;
+    half = 0;
+    guard = 0;
+    cy = f2i(floorf(y1));
+    bound = ceilf(y2);
+    if (y1 == y2 || !((float)cy <= bound)) top();
+  }
+  __device__ __forceinline__ void top() {
+    half = 1;
+    s1 = (x3 - x2) / (y3 - y2);
+    s2 = (x3 - x4) / (y3 - y2);
+    cx1 = x3; cx2 = x3;
+    if (s1 < s2) swap_(s1, s2);
+    sbias = y3 - floorf(y3);
+    cy = f2i(ceilf(y3));
+    bound = floorf(y2);
+    if (y2 == y3 || !((float)cy >= bound) || guard >= 2 * LOOP_LIMIT) half = 2;
+  }
+  __device__ __forceinline__ bool done() const { return half == 2; }
+  // the current row's tiles [first, first + n); then to the next row
+  __device__ __forceinline__ void row(int &first, int &n) {
+    const float dir = half == 0 ? 1.f : -1.f;          // products with -1 and a + (-b) are exact
+    float mx1 = cx1 + dir * (sbias * s1), mx2 = cx2 + dir * (sbias * s2);
+    if (s1 < 0) mx1 -= dir * s1;
+    if (s2 > 0) mx2 -= dir * s2;
+    const float hi = fminf(half == 0 ? mx1 : mx2, wcm1), lo = fmaxf(half == 0 ? mx2 : mx1, 0.f);
+    n = 0;
+    first = 0;
+    if (cy >= 0 && cy < hc) {
+      int a1 = f2i(floorf(lo));
+      float hb = ceilf(hi);                            // at most wc - 1
+      if ((float)a1 <= hb) n = f2i(hb) - a1 + 1;
+      first = wc * cy + a1;
+    }
+    cx1 += dir * s1;
+    cx2 += dir * s2;
+    guard++;
+    if (half == 0) {
+      cy++;
+      if (!((float)cy <= bound) || guard >= LOOP_LIMIT) top();
+    } else {
+      cy--;
+      if (!((float)cy >= bound) || guard >= 2 * LOOP_LIMIT) half = 2;
     }
   }
-  s1 = (x3 - x2) / (y3 - y2);
-  s2 = (x3 - x4) / (y3 - y4);
-  cx1 = x3; cx2 = x3;
-  if (s1 < s2) { t = s1; s1 = s2; s2 = t; }
-  sbias = y3 - floorf(y3);
-  if (y2 != y3) {
-    for (int cy = f2i(ceilf(y3)); (float)cy >= floorf(y2) && guard < 2 * LOOP_LIMIT; cy--, guard++) {
-      float mx1 = cx1 - sbias * s1;
-      if (s1 < 0) mx1 += s1;
-      float mx2 = cx2 - sbias * s2;
-      if (s2 > 0) mx2 += s2;
-      mx2 = fminf(mx2, wcm1);
-      mx1 = fmaxf(mx1, 0.f);
-      if (cy >= 0 && cy < hc) {
-        int a1 = f2i(floorf(mx1));
-        float hb = ceilf(mx2);
-        for (int ax = a1; (float)ax <= hb && ax < wc; ax++) emit(wc * cy + ax);
-      }
-      cx1 -= s1;
-      cx2 -= s2;
-    }
+};
+// calls emit(tile) for every bin entry
+template <class F>
+__device__ __forceinline__ void coarse_walk(const float sx[3], const float sy[3], int wc, int hc, F emit) {
+  CoarseWalk W;
+  W.init(sx, sy, wc, hc);
+  while (!W.done()) {
+    int first, n;
+    W.row(first, n);
+    for (int k = 0; k < n; k++) emit(first + k);
   }
 }
 
-// Opaque units fill the queue from the front, alpha-tested ones from the back.
+// Opaque units fill the queue from the front, alpha-tested ones from the
+// back.  A lane walks its triangle's tile rows twice: to count its units (a row's
+// number is known without walking its tiles), and, once the queue's room is
+// reserved, row by row with the others, the warp writing each row's units
+// together.  Walking every tile twice on its own lane took 30 us for the 4,329
+// large triangles of the 1080p frame, this 23 us; 4 lanes a claim instead of as few
+// as one saves instructions and not time.
 __device__ __forceinline__ void coarse_loop(const DrawParams &P, const GroupDev *sg, int lane) {
   uint32_t n = P.ctr[CTR_LARGE];
   int wc = P.view.w / TILE, hc = P.view.h / TILE;
@@ -1352,16 +1370,24 @@ __device__ __forceinline__ void coarse_loop(const DrawParams &P, const GroupDev 
     base = __shfl_sync(FULL, base, 0);
     if (base >= n) break;
     bool live = (uint32_t)lane < per && base + lane < n;
-    float sx[3], sy[3], sz[3];
+    CoarseWalk start;
+    start.half = 2;
     uint32_t gt = 0;
     int cnt = 0;
     bool alpha = false;
     if (live) {
+      float sx[3], sy[3], sz[3];
       gt = P.large_list[base + lane];
       const GroupDev &G = sg[find_group(sg, P.ngroups, gt)];
       alpha = (G.flags & F_ALPHA) != 0;
       project_persp(G, (int)(gt - G.tri_base), P.view, sx, sy, sz);
-      coarse_walk(sx, sy, wc, hc, [&](int) { cnt++; });
+      start.init(sx, sy, wc, hc);
+      CoarseWalk W = start;
+      while (!W.done()) {
+        int first, m;
+        W.row(first, m);
+        cnt += m;
+      }
     }
     int co = alpha ? 0 : cnt, ca = alpha ? cnt : 0;
     int io = co, ia = ca;
@@ -1387,19 +1413,22 @@ __device__ __forceinline__ void coarse_loop(const DrawParams &P, const GroupDev 
       }
     }
     fits = __shfl_sync(FULL, fits, 31);
+    if (!fits) continue;
     oo = __shfl_sync(FULL, oo, 31) + (uint32_t)(io - co);
     oa = __shfl_sync(FULL, oa, 31) + (uint32_t)(ia - ca);
-    if (live && cnt && fits) {
-      {
-        int k = 0;
-        if (!alpha) {
-          uint2 *u = P.units + oo;
-          coarse_walk(sx, sy, wc, hc, [&](int tile) { u[k++] = make_uint2(gt, (uint32_t)tile); });
-        } else {
-          uint2 *u = P.units + (P.cap_units - 1 - oa);
-          coarse_walk(sx, sy, wc, hc, [&](int tile) { *(u - k) = make_uint2(gt, (uint32_t)tile); k++; });
-        }
+    // position of the lane's next unit, and whether positions run downwards
+    uint32_t at = alpha ? P.cap_units - 1 - oa : oo;
+    while (__any_sync(FULL, !start.done())) {
+      int first = 0, m = 0;
+      if (!start.done()) start.row(first, m);
+      for (unsigned todo = __ballot_sync(FULL, m > 0); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        const int f = __shfl_sync(FULL, first, src), c = __shfl_sync(FULL, m, src);
+        const uint32_t p = __shfl_sync(FULL, at, src), g = __shfl_sync(FULL, gt, src);
+        const bool down = __shfl_sync(FULL, (int)alpha, src) != 0;
+        for (int k = lane; k < c; k += 32) P.units[down ? p - k : p + k] = make_uint2(g, (uint32_t)(f + k));
       }
+      at = alpha ? at - m : at + m;
     }
   }
 }
@@ -1677,9 +1706,6 @@ __device__ __forceinline__ float shadow_light(const DrawParams &P, V3 p) {
   float light = (float)shadow * P.light.amb + (float)(5 - shadow);
   return light * 0.2f;
 }
-
-template <class A>
-__device__ __forceinline__ void swap_(A &a, A &b) { A t = a; a = b; b = t; }
 
 // One edge chain of a triangle half on some row: x, 1/depth and the attributes
 // (times 1/depth).

@@ -59,6 +59,9 @@ struct LightDev {
 
 // ------------------------------------------------------------ scalars
 
+template <class A>
+__device__ __forceinline__ void swap_(A &a, A &b) { A t = a; a = b; b = t; }
+
 __device__ __forceinline__ int f2i(float x) { return __float2int_rz(x); }
 // t = max(0, min(1, t)) with min/max = fminf/fmaxf, so NaN (0/0 on one-pixel
 // spans) gives 1.  Written with an explicit NaN branch because the compiler
@@ -242,6 +245,17 @@ template <bool FULL> __device__ __forceinline__ Attr<FULL> a_load(const GroupDev
 
 // ------------------------------------------------------------ setup
 
+// The reciprocals of three depths, without the division's special cases when
+// all lie in the ordinary range.
+__device__ __forceinline__ void recip3(float d[3]) {
+  float a = fabsf(d[0]), b = fabsf(d[1]), c = fabsf(d[2]);
+  if (a >= 0x1p-60f && a <= 0x1p60f && b >= 0x1p-60f && b <= 0x1p60f && c >= 0x1p-60f && c <= 0x1p60f) {
+    d[0] = recip_rn(d[0]); d[1] = recip_rn(d[1]); d[2] = recip_rn(d[2]);
+  } else {
+    d[0] = 1.0f / d[0]; d[1] = 1.0f / d[1]; d[2] = 1.0f / d[2];
+  }
+}
+
 // trisetup.c:29-80 / trisetup_cull.c:49-54: returns 0 rejected, 1 small, 2 large
 __device__ __forceinline__ int project_persp(const GroupDev &g, int tri, const ViewDev &v, float sx[3], float sy[3],
                                              float sz[3]) {
@@ -257,9 +271,9 @@ __device__ __forceinline__ int project_persp(const GroupDev &g, int tri, const V
     dx[k] = dot3(x[k], svx);
     dy[k] = dot3(x[k], svy);
   }
+  recip3(dd);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    dd[k] = 1.0f / dd[k];
     dx[k] = dx[k] * dd[k];
     dy[k] = dy[k] * dd[k];
   }
@@ -300,18 +314,14 @@ __device__ __forceinline__ bool project_ortho(const GroupDev &g, int tri, const 
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     V3 x = sub3(ld3(p + 3 * k), vp);
-    float dd = dot3(x, svd);
-    float dx = dot3(x, svx);
-    float dy = dot3(x, svy);
-    dd = dd + bias;
-    dd = 1.0f / dd;
-    dx = dx * s.scale + half;
-    dy = dy * -s.scale + half;
-    ix[k] = f2i(dx);
-    iy[k] = f2i(dy);
-    z[k] = dd;
-    if (!(dd > 0) || ix[k] < -120 || ix[k] >= s.dim + 120 || iy[k] < -120 || iy[k] >= s.dim + 120) yes = false;
+    z[k] = dot3(x, svd) + bias;
+    ix[k] = f2i(dot3(x, svx) * s.scale + half);
+    iy[k] = f2i(dot3(x, svy) * -s.scale + half);
   }
+  recip3(z);
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    if (!(z[k] > 0) || ix[k] < -120 || ix[k] >= s.dim + 120 || iy[k] < -120 || iy[k] >= s.dim + 120) yes = false;
   return yes;
 }
 
