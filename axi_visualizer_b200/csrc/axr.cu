@@ -71,7 +71,7 @@ struct Alpha {
 // A shadow map has its own stream, scratch (caster list, counters) and group
 // table, so cascades render concurrently with each other and with the main
 // view's visibility pass; ev_write orders the shade pass after the map's last
-// writer, ev_read orders the next writer after the map's last reader.
+// writer, `reader` the next writer after the map's last reader.
 struct Shadow {
   float *map = nullptr;
   int dim = 0;
@@ -80,12 +80,21 @@ struct Shadow {
   float vv[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
   cudaStream_t st = nullptr;
   cudaEvent_t ev_write = nullptr, ev_read = nullptr;
+  // The event after the map's last reader, and counts of what was recorded
+  // and what the other side has waited for: an event waited for once is not
+  // waited for again (the order of a stream's work stays).
+  cudaEvent_t reader = nullptr;
+  uint64_t write_seq = 0, write_waited = 0, read_seq = 0, read_waited = 0, geo_waited = 0;
   uint32_t *list = nullptr, *ctr = nullptr, *items = nullptr;
   uint32_t cap = 0;          // casters the list (and the records) hold
   bool items_ready = false;  // row-chunk items allocated (per-caster path)
   GroupDev *tab = nullptr;
+  // two sets of counters, used in turn: a pass's setup clears the other set
+  // for the next pass (clean), so that no memset stands before it
+  int cur = 0;
+  bool clean[2] = {false, false};
   // tiled pass: caster records, tile offsets/cursors/order, units; the
-  // per-tile counts sit right after the CTR_N counters (one clear for both)
+  // per-tile counts sit right after the two sets of counters
   uint4 *rec = nullptr;
   uint32_t *tiles = nullptr, *units = nullptr;
   uint32_t cap_units = 0;
@@ -102,6 +111,10 @@ struct Shadow {
 };
 
 constexpr int MAX_GROUPS = 64;
+// from this many triangles the alpha-tested rasterizers run on their own stream
+// (2,512 triangles at 320x192: 99 us a frame among others without, 107 with
+// it, alone 190 and 171; 301,000 at 720p: 452 alone without, 385 with it)
+constexpr int SIDE_STREAM_TRIS = 8192;
 constexpr int MAX_SHADOWS = 16;
 // 3 * ntris + 3 stays an int: the vertex kernels round v_end up to a quad
 constexpr int MAX_GROUP_TRIS = (INT_MAX - 3) / 3;
@@ -149,19 +162,11 @@ struct axr_ctx {
   } rd[2];
   cudaStream_t s_copy = nullptr;
   int64_t read_seq = 0;
-  // pinned staging of the per-call group tables: a host-to-device copy from
-  // pageable memory would first synchronise its stream, i.e. wait for the
-  // previous frame; a slot is reused only after the copy that read it ran
-  struct Stage {
-    GroupDev *h = nullptr;
-    cudaEvent_t ev = nullptr;
-    bool used = false;
-  } stage[8];
-  int stage_next = 0;
   // vertex stage: ev_geo follows the last geometry write on `stream`
   // (rotate/translate/copyTo), which shadow passes on their own streams wait
   // for; the light table of vertLight is staged through pinned memory
   cudaEvent_t ev_geo = nullptr;
+  uint64_t geo_seq = 0;
   float *d_lights = nullptr, *h_lights = nullptr;
   size_t lights_cap = 0;
   cudaEvent_t ev_lights = nullptr;
@@ -502,32 +507,48 @@ int group_table(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, co
   return 0;
 }
 
-// Copies a group table to the device on stream s through the pinned ring.
-int upload_table(axr_ctx *c, GroupDev *dst, const GroupDev *tab, int n, cudaStream_t s) {
-  axr_ctx::Stage &st = c->stage[c->stage_next];
-  c->stage_next = (c->stage_next + 1) % 8;
-  if (!st.h) {
-    if (cudaMallocHost(&st.h, sizeof(GroupDev) * MAX_GROUPS) != cudaSuccess) return fail(AXR_ENOMEM, "group table");
-    CK(cudaEventCreateWithFlags(&st.ev, cudaEventDisableTiming));
-  } else if (st.used) {
-    CK(cudaEventSynchronize(st.ev));
+// Calls f with the table as a kernel argument of 16 groups' size, or of 64
+template <class F>
+void with_table(const GroupDev *tab, int ngroups, F f) {
+  if (ngroups <= 16) {
+    GroupTab<16> t;
+    memcpy(t.g, tab, sizeof t.g);
+    f(t);
+  } else {
+    GroupTab<MAX_GROUPS> t;
+    memcpy(t.g, tab, sizeof t.g);
+    f(t);
   }
-  memcpy(st.h, tab, sizeof(GroupDev) * n);
-  CK(cudaMemcpyAsync(dst, st.h, sizeof(GroupDev) * n, cudaMemcpyHostToDevice, s));
-  CK(cudaEventRecord(st.ev, s));
-  st.used = true;
-  return 0;
 }
 
-// Builds the per-call group table on the device.
-int upload_groups(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, const uint8_t *enabled_mask,
-                  bool mask_means_enabled, int ngroups) {
-  GroupDev tab[MAX_GROUPS];
-  int rc = group_table(c, flags, alpha_index, enabled_mask, mask_means_enabled, ngroups, tab);
-  if (rc) return rc;
-  rc = upload_table(c, c->d_groups, tab, std::max(ngroups, 1), c->stream);
-  if (rc) return rc;
+// The handle's stream waits for a map's last writer; a map's stream for its
+// last reader, and for the last geometry write (rotate / translate / copyTo).
+int wait_writer(axr_ctx *c, Shadow &sm) {
+  if (sm.write_waited == sm.write_seq) return 0;
+  CK(cudaStreamWaitEvent(c->stream, sm.ev_write, 0));
+  sm.write_waited = sm.write_seq;
   return 0;
+}
+int wait_readers(Shadow &sm) {
+  if (sm.read_waited == sm.read_seq) return 0;
+  CK(cudaStreamWaitEvent(sm.st, sm.reader, 0));
+  sm.read_waited = sm.read_seq;
+  return 0;
+}
+int wait_geometry(axr_ctx *c, Shadow &sm) {
+  if (sm.geo_waited == c->geo_seq) return 0;
+  CK(cudaStreamWaitEvent(sm.st, c->ev_geo, 0));
+  sm.geo_waited = c->geo_seq;
+  return 0;
+}
+int wrote(Shadow &sm) {
+  CK(cudaEventRecord(sm.ev_write, sm.st));
+  sm.write_seq++;
+  return 0;
+}
+void read_until(Shadow &sm, cudaEvent_t e) {
+  sm.reader = e;
+  sm.read_seq++;
 }
 
 }  // namespace
@@ -645,10 +666,6 @@ int axr_destroy(axr_ctx *c) {
     if (r.done) cudaEventDestroy(r.done);
   }
   if (c->s_copy) { cudaStreamSynchronize(c->s_copy); cudaStreamDestroy(c->s_copy); }
-  for (auto &st : c->stage) {
-    if (st.ev) { cudaEventSynchronize(st.ev); cudaEventDestroy(st.ev); }
-    if (st.h) cudaFreeHost(st.h);
-  }
   for (auto &p : c->tpend) { c->ev_pool.push_back(p.a); c->ev_pool.push_back(p.b); }
   for (auto e : c->ev_pool) cudaEventDestroy(e);
   if (c->ev_geo) cudaEventDestroy(c->ev_geo);
@@ -792,11 +809,12 @@ namespace {
 // `body` has queued the write, marks it for the next shadow passes.
 template <class F>
 int geometry_write(axr_ctx *c, F body) {
+  int rc = 0;
   for (auto &sm : c->shadows)
-    if (sm.st) CK(cudaStreamWaitEvent(c->stream, sm.ev_write, 0));
-  int rc = body();
-  if (rc) return rc;
+    if (sm.st && (rc = wait_writer(c, sm))) return rc;
+  if ((rc = body())) return rc;
   CK(cudaEventRecord(c->ev_geo, c->stream));
+  c->geo_seq++;
   return 0;
 }
 
@@ -1006,7 +1024,9 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
     memcpy(P.sh[k].vv, s.vv, sizeof s.vv);
   }
   if (any_shadow && nshadow == 0) return fail(AXR_ESTATE, "shadow materials drawn with no shadow map");
-  if ((rc = upload_groups(c, flags, alpha_index, mask, false, ngroups))) return rc;
+  GroupDev tab[MAX_GROUPS];
+  if ((rc = group_table(c, flags, alpha_index, mask, false, ngroups, tab))) return rc;
+  const int slot = 1 - c->last_slot;
   P.groups = c->d_groups;
   P.ngroups = ngroups;
   P.total_tris = c->total_tris;
@@ -1020,48 +1040,59 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
   P.cap_list = c->cap_list; P.cap_units = c->cap_units;
   P.min_chunk = c->min_chunk;
   P.claim_k = 1;
+  P.host_ctr = c->h_ring + slot * CTR_N;
   long npix = (long)c->w * c->h;
   cudaStream_t s = c->stream;
   int64_t nk = 0;
-  cudaStream_t sa = c->s_alpha;
-  launch(c, s, "k_init_keys", [&] { k_init_keys<<<grid_for(c, npix, 256, 16), 256, 0, s>>>(c->db, c->keys, (int)npix, c->ctr); }); nk++;
+  const bool side = any_alpha && c->total_tris >= SIDE_STREAM_TRIS;
+  cudaStream_t sa = side ? c->s_alpha : s;
+  with_table(tab, ngroups, [&](const auto &t) {
+    launch(c, s, "k_init_keys", [&] {
+      k_init_keys<<<grid_for(c, npix, 256, 16), 256, 0, s>>>(c->db, c->keys, (int)npix, c->ctr, t, c->d_groups, ngroups);
+    });
+  });
+  nk++;
   if (c->total_tris > 0) {
     // visibility: opaque rasterizers on the main stream, alpha-tested ones
     // concurrently on a side stream (all of them atomicMin the same buffer)
     launch(c, s, "k_setup", [&] { k_setup<<<grid_for(c, c->total_tris, SETUP_THREADS, 8), SETUP_THREADS, 0, s>>>(P); }); nk++;
-    if (any_alpha) {
+    if (side) {
       CK(cudaEventRecord(c->ev_setup, s));
       CK(cudaStreamWaitEvent(sa, c->ev_setup, 0));
+    }
+    if (any_alpha) {
       launch(c, sa, "k_raster_small_alpha", [&] { k_raster_small<true><<<c->sms * c->occ[1], 128, 0, sa>>>(P); }); nk++;
     }
     launch(c, s, "k_raster_small", [&] { k_raster_small<false><<<c->sms * c->occ[0], 128, 0, s>>>(P); }); nk++;
     launch(c, s, "k_coarse", [&] { k_coarse<<<c->sms * 4, 128, 0, s>>>(P); }); nk++;
-    if (any_alpha) {
+    if (side) {
       CK(cudaEventRecord(c->ev_coarse, s));
       CK(cudaStreamWaitEvent(sa, c->ev_coarse, 0));
+    }
+    if (any_alpha) {
       launch(c, sa, "k_raster_tiled_alpha", [&] { k_raster_tiled<true><<<c->sms * c->occ[3], 128, 0, sa>>>(P); }); nk++;
     }
     launch(c, s, "k_raster_tiled", [&] { k_raster_tiled<false><<<c->sms * c->occ[2], 128, 0, s>>>(P); }); nk++;
     launch(c, s, "k_raster_tiled_fallback", [&] { k_raster_tiled_fallback<<<c->sms * 2, 128, 0, s>>>(P); }); nk++;
-    if (any_alpha) {
+    if (side) {
       CK(cudaEventRecord(c->ev_alpha, sa));
       CK(cudaStreamWaitEvent(s, c->ev_alpha, 0));
     }
   }
   // shading samples the cascades: wait for their last writers
-  for (int k = 0; k < nshadow; k++) CK(cudaStreamWaitEvent(s, c->shadows[shadow_ids[k]].ev_write, 0));
+  for (int k = 0; k < nshadow; k++)
+    if ((rc = wait_writer(c, c->shadows[shadow_ids[k]]))) return rc;
+  // the shade writes the counters over those of the frame before last
+  if (c->pend[slot] && (rc = check_slot(c, slot, true))) return rc;
   dim3 sb(256), sgd((c->w + 15) / 16, (c->h + 15) / 16);   // a 16x16 tile per block
   if (any_normal)
     launch(c, s, "k_shade", [&] { k_shade<true><<<sgd, sb, 0, s>>>(P); });
   else
     launch(c, s, "k_shade", [&] { k_shade<false><<<sgd, sb, 0, s>>>(P); });
   nk++;
-  for (int k = 0; k < nshadow; k++) CK(cudaEventRecord(c->shadows[shadow_ids[k]].ev_read, s));
   CK(cudaGetLastError());
-  int slot = 1 - c->last_slot;
-  if (c->pend[slot] && (rc = check_slot(c, slot, true))) return rc;   // the frame before last
-  CK(cudaMemcpyAsync(c->h_ring + slot * CTR_N, c->ctr, sizeof(uint32_t) * CTR_N, cudaMemcpyDeviceToHost, s));
   CK(cudaEventRecord(c->ev_ctr[slot], s));
+  for (int k = 0; k < nshadow; k++) read_until(c->shadows[shadow_ids[k]], c->ev_ctr[slot]);
   c->pend[slot] = true;
   c->last_slot = slot;
   c->last_kernels = nk;
@@ -1294,17 +1325,18 @@ int axr_add_shadow_map(axr_ctx *c, int i, int size, float scale, float amb) {
     cudaFree(s.map); cudaFree(s.ctr); cudaFree(s.tiles);
     s.map = nullptr; s.ctr = s.tiles = nullptr;
   }
-  CK(cudaStreamWaitEvent(s.st, s.ev_read, 0));
+  if ((rc = wait_readers(s))) return rc;
   if (!s.map) {
-    // counters, then the per-tile unit counts and claim counters of the
+    // two sets of counters, then the per-tile unit counts and claim counters of the
     // tiled pass (opaque, alpha); tile offsets, cursors (2 per tile), order
     // and the prefix of blocks per tile
     s.ntx = (size + STILE - 1) / STILE;
     size_t nt = (size_t)s.ntx * s.ntx;
     if (cudaMalloc(&s.map, sizeof(float) * (size_t)size * size) != cudaSuccess ||
-        cudaMalloc(&s.ctr, sizeof(uint32_t) * (CTR_N + 4 * nt)) != cudaSuccess ||
+        cudaMalloc(&s.ctr, sizeof(uint32_t) * (2 * CTR_N + 4 * nt)) != cudaSuccess ||
         cudaMalloc(&s.tiles, sizeof(uint32_t) * (5 * nt + 1)) != cudaSuccess)
       return fail(AXR_ENOMEM, "shadow map %dx%d", size, size);
+    s.clean[0] = s.clean[1] = false;
   }
   s.dim = size;
   s.scale = scale;
@@ -1312,7 +1344,7 @@ int axr_add_shadow_map(axr_ctx *c, int i, int size, float scale, float amb) {
   k_clear_depth<<<grid_for(c, (long)size * size, 256, 8), 256, 0, s.st>>>(s.map, size, size, 1);
   c->launches++;
   CK(cudaGetLastError());
-  CK(cudaEventRecord(s.ev_write, s.st));
+  if ((rc = wrote(s))) return rc;
   c->amb = amb;
   return 0;
 }
@@ -1331,10 +1363,10 @@ int axr_clear_shadow_map(axr_ctx *c, int i) {
   if (rc) return rc;
   if (i < 0 || i >= MAX_SHADOWS || !c->shadows[i].map) return fail(AXR_ESTATE, "shadow map %d does not exist", i);
   Shadow &s = c->shadows[i];
-  CK(cudaStreamWaitEvent(s.st, s.ev_read, 0));
+  if ((rc = wait_readers(s))) return rc;
   launch(c, s.st, "k_clear_shadow", [&] { k_clear_depth<<<grid_for(c, (long)s.dim * s.dim, 256, 8), 256, 0, s.st>>>(s.map, s.dim, s.dim, 16); });
   CK(cudaGetLastError());
-  CK(cudaEventRecord(s.ev_write, s.st));
+  if ((rc = wrote(s))) return rc;
   return 0;
 }
 
@@ -1344,7 +1376,7 @@ int axr_shadow_map(axr_ctx *c, int i, const uint8_t *cast, const int32_t *flags,
   if (rc) return rc;
   if (i < 0 || i >= MAX_SHADOWS || !c->shadows[i].map) return fail(AXR_ESTATE, "shadow map %d does not exist", i);
   if (ngroups != (int)c->groups.size() || !cast) return fail(AXR_EINVAL, "shadowMap arguments");
-  if ((rc = settle_next(c))) return rc;
+  if (!c->tpend.empty() && (rc = settle(c))) return rc;   // (with per-kernel timing)
   // alpha casters use the alpha mask's own side as lenT (drawminalpha.c:86-96)
   std::vector<int32_t> fl(ngroups, 0);
   for (int g = 0; g < ngroups; g++) fl[g] = flags ? (flags[g] & (F_ALPHA | F_MIP)) : 0;
@@ -1393,22 +1425,20 @@ int axr_shadow_map(axr_ctx *c, int i, const uint8_t *cast, const int32_t *flags,
       return fail(AXR_ENOMEM, "row chunks of shadow map %d", i);
     sm.items_ready = true;
   }
-  CK(cudaStreamWaitEvent(sm.st, sm.ev_read, 0));
-  CK(cudaStreamWaitEvent(sm.st, c->ev_geo, 0));   // rotate / translate / copyTo queued before
-  if ((rc = upload_table(c, sm.tab, tab, std::max(ngroups, 1), sm.st))) return rc;
+  if ((rc = wait_readers(sm)) || (rc = wait_geometry(c, sm))) return rc;
   ShadowParams S;
   memset(&S, 0, sizeof S);
   S.groups = sm.tab; S.ngroups = ngroups; S.total_tris = c->total_tris;
   S.sh.map = sm.map; S.sh.dim = sm.dim; S.sh.scale = sm.scale;
   memcpy(S.sh.pos, sm.pos, sizeof sm.pos);
   memcpy(S.sh.vv, sm.vv, sizeof sm.vv);
-  S.map = sm.map; S.bias = bias; S.list = sm.list; S.cap_list = sm.cap; S.ctr = sm.ctr;
+  S.map = sm.map; S.bias = bias; S.list = sm.list; S.cap_list = sm.cap;
   S.min_chunk = c->min_chunk;
   S.claim_k = 1;
   const size_t nt = (size_t)sm.ntx * sm.ntx;
   if (tiled) {
     S.rec = sm.rec;
-    S.tcnt = sm.ctr + CTR_N; S.tclaim = sm.ctr + CTR_N + 2 * nt;
+    S.tcnt = sm.ctr + 2 * CTR_N; S.tclaim = sm.ctr + 2 * CTR_N + 2 * nt;
     S.toff = sm.tiles; S.tcur = sm.tiles + nt; S.tord = sm.tiles + 3 * nt; S.hpre = sm.tiles + 4 * nt;
     S.units = sm.units; S.cap_units = sm.cap_units;
     S.ntx = sm.ntx; S.ntiles = (int)nt;
@@ -1422,9 +1452,18 @@ int axr_shadow_map(axr_ctx *c, int i, const uint8_t *cast, const int32_t *flags,
     if (cast[g] && (tab[g].flags & F_ALPHA)) any_alpha = true;
   static_assert(CTR_SH_LIST_A == CTR_SH_LIST + 1 && CTR_SH_WORK == CTR_SH_LIST + 2 && CTR_SH_WORK_A == CTR_SH_LIST + 3,
                 "shadow counters are contiguous");
-  CK(cudaMemsetAsync(sm.ctr, 0, sizeof(uint32_t) * (CTR_N + (tiled ? 4 * nt : 0)), sm.st));
+  sm.cur = 1 - sm.cur;
+  S.ctr = sm.ctr + sm.cur * CTR_N;
+  S.zero = sm.ctr + (1 - sm.cur) * CTR_N;
+  if (!sm.clean[sm.cur]) CK(cudaMemsetAsync(S.ctr, 0, sizeof(uint32_t) * CTR_N, sm.st));
+  sm.clean[sm.cur] = false;
+  if (tiled) CK(cudaMemsetAsync(S.tcnt, 0, sizeof(uint32_t) * 4 * nt, sm.st));
   cudaStream_t st = sm.st;
-  launch(c, st, "k_shadow_setup", [&] { k_shadow_setup<<<grid_for(c, c->total_tris, 256, 16), 256, 0, st>>>(S); });
+  with_table(tab, ngroups, [&](const auto &t) {
+    launch(c, st, "k_shadow_setup",
+           [&] { k_shadow_setup<<<grid_for(c, c->total_tris, 256, 16), 256, 0, st>>>(S, t, sm.tab); });
+  });
+  sm.clean[1 - sm.cur] = true;
   if (tiled) {
     launch(c, st, "k_shadow_scan", [&] { k_shadow_scan<<<1, SCAN_THREADS, 0, st>>>(S); });
     launch(c, st, "k_shadow_bin", [&] { k_shadow_bin<<<c->sms * 8, 256, 0, st>>>(S); });
@@ -1438,11 +1477,11 @@ int axr_shadow_map(axr_ctx *c, int i, const uint8_t *cast, const int32_t *flags,
       launch(c, st, "k_shadow_raster_alpha", [&] { k_shadow_raster<true><<<c->sms * c->occ[5], 128, 0, st>>>(S); });
   }
   CK(cudaGetLastError());
-  CK(cudaEventRecord(sm.ev_write, st));
+  if ((rc = wrote(sm))) return rc;
   // the pass's counters to the ring (the slot before last is checked first)
-  int slot = 1 - sm.last_slot;
+  const int slot = 1 - sm.last_slot;
   if (sm.pend[slot] && (rc = check_shadow_slot(sm, slot, true))) return rc;
-  CK(cudaMemcpyAsync(sm.h_ring + slot * CTR_N, sm.ctr, sizeof(uint32_t) * CTR_N, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(sm.h_ring + slot * CTR_N, S.ctr, sizeof(uint32_t) * CTR_N, cudaMemcpyDeviceToHost, st));
   CK(cudaEventRecord(sm.ev_ctr[slot], st));
   sm.pend[slot] = true;
   sm.last_slot = slot;
@@ -1976,7 +2015,7 @@ int axr_batch_render(axr_batch *b, const int32_t *flags, const int32_t *alpha_in
   // shaded views sampling the handle's own shadow maps wait for their writers
   for (auto &v : b->desc)
     for (int j = 0; j < v.ncascades; j++)
-      if (v.cascades[j] < 0) CK(cudaStreamWaitEvent(c->stream, c->shadows[-1 - v.cascades[j]].ev_write, 0));
+      if (v.cascades[j] < 0 && (rc = wait_writer(c, c->shadows[-1 - v.cascades[j]]))) return rc;
   // the framebuffers are free once the last render's read-back has left them
   if (b->reads) CK(cudaStreamWaitEvent(c->stream, b->read_done, 0));
   b->reads = false;
@@ -1993,7 +2032,11 @@ int axr_batch_render(axr_batch *b, const int32_t *flags, const int32_t *alpha_in
   // the handle's shadow maps this render sampled: it is their last reader
   for (auto &v : b->desc)
     for (int j = 0; j < v.ncascades; j++)
-      if (v.kind == AXR_VIEW_SHADED && v.cascades[j] < 0) CK(cudaEventRecord(c->shadows[-1 - v.cascades[j]].ev_read, c->stream));
+      if (v.kind == AXR_VIEW_SHADED && v.cascades[j] < 0) {
+        Shadow &sm = c->shadows[-1 - v.cascades[j]];
+        CK(cudaEventRecord(sm.ev_read, c->stream));
+        read_until(sm, sm.ev_read);
+      }
   CK(cudaEventRecord(b->done, c->stream));
   b->pending = true;
   return 0;

@@ -43,6 +43,7 @@ struct DrawParams {
   uint32_t cap_list, cap_units;
   int min_chunk;         // rows per small-triangle work item (at least; tuning knob)
   int claim_k;           // claim_size's k for the short queues (0: 32 items per claim)
+  uint32_t *host_ctr;    // pinned host copy of the counters, written by the shade; null: none
 };
 
 enum {
@@ -119,9 +120,26 @@ __device__ __forceinline__ int chunk_len(int rows, int min_chunk) {
 
 // ------------------------------------------------------------ keys / clear
 
-__global__ void k_init_keys(const float *__restrict__ db, uint64_t *__restrict__ keys, int n, uint32_t *ctr) {
+// A draw's or pass's group table as a kernel argument: the first kernel of the
+// chain writes it to the device table that the later ones read, so that no
+// host-to-device copy (and no staging buffer to wait for) stands before them.
+template <int N>
+struct GroupTab {
+  GroupDev g[N];
+};
+template <int N>
+__device__ __forceinline__ void store_table(const GroupTab<N> &tab, GroupDev *dst, int ngroups) {
+  const uint32_t *src = reinterpret_cast<const uint32_t *>(tab.g);
+  uint32_t *d = reinterpret_cast<uint32_t *>(dst);
+  for (int i = threadIdx.x; i < ngroups * (int)(sizeof(GroupDev) / 4); i += blockDim.x) d[i] = src[i];
+}
+
+template <int N>
+__global__ void k_init_keys(const float *__restrict__ db, uint64_t *__restrict__ keys, int n, uint32_t *ctr,
+                            const __grid_constant__ GroupTab<N> tab, GroupDev *dst, int ngroups) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < CTR_N && blockIdx.x == 0) ctr[i] = 0;
+  if (blockIdx.x == 0) store_table(tab, dst, ngroups);
   for (; i < n; i += gridDim.x * blockDim.x) keys[i] = ((uint64_t)depth_key(db[i]) << 32) | 0xffffffffull;
 }
 
@@ -2193,6 +2211,8 @@ __global__ void __launch_bounds__(256, 4) k_shade(DrawParams P) {   // 64 regist
   __shared__ GroupDev sg[64];
   __shared__ ShadeSmem<256> sm;
   for (int i = threadIdx.x; i < P.ngroups; i += blockDim.x) sg[i] = P.groups[i];
+  if (P.host_ctr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < CTR_N)
+    P.host_ctr[threadIdx.x] = P.ctr[threadIdx.x];     // final: every kernel that counts has finished
   __syncthreads();
   shade_tile<256, NRM>(P, sg, blockIdx.x * TILE, blockIdx.y * TILE, sm);
 }
@@ -2218,6 +2238,7 @@ struct ShadowParams {
   uint32_t *list;      // opaque casters from the front, alpha-tested from the back
   uint32_t cap_list;
   uint32_t *ctr;
+  uint32_t *zero;      // the next pass's counters, cleared by this one's setup; null: none
   uint32_t *items;     // row chunks of the casters, same two ends (cap_list * MAX_CHUNKS);
                        // null: one work item per caster
   int min_chunk;       // rows per chunk (at least)
@@ -2366,9 +2387,15 @@ __device__ __forceinline__ void shadow_setup_phase(const ShadowParams &S, const 
   }
 }
 
-__global__ void __launch_bounds__(256) k_shadow_setup(ShadowParams S) {
-  __shared__ GroupDev sg[64];
-  for (int i = threadIdx.x; i < S.ngroups; i += blockDim.x) sg[i] = S.groups[i];
+template <int N>
+__global__ void __launch_bounds__(256, 6) k_shadow_setup(ShadowParams S, const __grid_constant__ GroupTab<N> tab,
+                                                      GroupDev *dst) {
+  __shared__ GroupDev sg[N];
+  for (int i = threadIdx.x; i < S.ngroups; i += blockDim.x) sg[i] = tab.g[i];
+  if (blockIdx.x == 0) {
+    store_table(tab, dst, S.ngroups);
+    if (S.zero && threadIdx.x < CTR_N) S.zero[threadIdx.x] = 0;
+  }
   __syncthreads();
   shadow_setup_phase(S, sg, blockIdx.x * blockDim.x, gridDim.x * blockDim.x);
 }
