@@ -115,6 +115,14 @@ constexpr int MAX_GROUPS = 64;
 // (2,512 triangles at 320x192: 99 us a frame among others without, 107 with
 // it, alone 190 and 171; 301,000 at 720p: 452 alone without, 385 with it)
 constexpr int SIDE_STREAM_TRIS = 8192;
+// Rows per work item where no tuning is set: 20 for casters, and for the small
+// triangles of large scenes, 12 (MIN_CHUNK) for those of others.  Setting an
+// item up costs as much as several rows, so fewer and longer items save
+// instructions; shorter ones spread a small view's work over more warps.  With 12
+// throughout the 4K / 2.9M-triangle frame took 2149 us, casters at 20 2043, both
+// 2019; 1080p / 1.04M 813, 798, 790; 720p / 300k 292, 287, 285, but alone 382,
+// 382, 397, and the normal-mapped 1296x713 view 157, 157, 165.
+constexpr int LONG_ITEM = 20, LONG_ITEM_TRIS = 700000;
 constexpr int MAX_SHADOWS = 16;
 // 3 * ntris + 3 stays an int: the vertex kernels round v_end up to a quad
 constexpr int MAX_GROUP_TRIS = (INT_MAX - 3) / 3;
@@ -177,7 +185,7 @@ struct axr_ctx {
   int light_blocks = 4;                      // resident 256-thread blocks of k_vert_light per SM
   // launch accounting and optional per-kernel CUDA-event timing
   int64_t launches = 0;
-  int min_chunk = MIN_CHUNK;
+  int min_chunk = 0;                         // rows per work item set by axr_set_tuning (0: by the scene's size)
   // resident blocks per SM of the persistent rasterizers (their grids are
   // one full wave): small opaque / alpha, tiled opaque / alpha, casters
   // opaque / alpha
@@ -1038,7 +1046,7 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
   P.small_list = c->small_list; P.large_list = c->large_list; P.items = c->items;
   P.units = c->units; P.ctr = c->ctr;
   P.cap_list = c->cap_list; P.cap_units = c->cap_units;
-  P.min_chunk = c->min_chunk;
+  P.min_chunk = c->min_chunk ? c->min_chunk : c->total_tris >= LONG_ITEM_TRIS ? LONG_ITEM : MIN_CHUNK;
   P.claim_k = 1;
   P.host_ctr = c->h_ring + slot * CTR_N;
   long npix = (long)c->w * c->h;
@@ -1433,7 +1441,7 @@ int axr_shadow_map(axr_ctx *c, int i, const uint8_t *cast, const int32_t *flags,
   memcpy(S.sh.pos, sm.pos, sizeof sm.pos);
   memcpy(S.sh.vv, sm.vv, sizeof sm.vv);
   S.map = sm.map; S.bias = bias; S.list = sm.list; S.cap_list = sm.cap;
-  S.min_chunk = c->min_chunk;
+  S.min_chunk = c->min_chunk ? c->min_chunk : LONG_ITEM;
   S.claim_k = 1;
   const size_t nt = (size_t)sm.ntx * sm.ntx;
   if (tiled) {
