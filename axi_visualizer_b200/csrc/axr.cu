@@ -606,7 +606,7 @@ int axr_create(int w, int h, int device, axr_ctx **out) {
       cudaEventCreateWithFlags(&c->ev_lights, cudaEventDisableTiming) != cudaSuccess) {
     rc = fail(AXR_ENOMEM, "framebuffers for %dx%d", w, h);
   }
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->light_blocks, k_vert_light, 256, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->light_blocks, k_vert_light<4, 4>, 256, 0);
   if (c->light_blocks < 1) c->light_blocks = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->ssao_blocks, k_ssao, 256, 0);
   if (c->ssao_blocks < 1) c->ssao_blocks = 1;
@@ -791,18 +791,26 @@ int axr_vert_light(axr_ctx *c, const uint8_t *mask, int ngroups, const float *di
   L.dint = d + off[0]; L.ddir = d + off[1]; L.pint = d + off[2]; L.ppos = d + off[3];
   L.sint = d + off[4]; L.sdir = d + off[5]; L.spos = d + off[6];
   L.nd = ndirs; L.np = npoints; L.ns = nspots; L.amb = amb;
-  VertJobs J;
+  VertJob jobs[MAX_GROUPS];
   int nj = 0, most = 0;
   for (int g = 0; g < ngroups; g++) {
     const Group &G = c->groups[g];
     if ((mask && !mask[g]) || !G.ntris) continue;
-    J.g[nj++] = {G.xyz, G.vn, G.li, G.ntris * 3};
+    jobs[nj++] = {G.xyz, G.vn, G.li, G.ntris * 3};
     most = std::max(most, G.ntris * 3);
   }
-  if (nj)
+  auto light = [&](auto J) {
+    constexpr int G = sizeof J.g / sizeof J.g[0];
+    std::copy(jobs, jobs + nj, J.g);
     launch(c, c->stream, "k_vert_light", [&] {
-      k_vert_light<<<dim3(grid_for(c, most / 4 + 1, 256, c->light_blocks), nj), 256, 0, c->stream>>>(J, L);
+      if (most >= c->sms * 1024)
+        k_vert_light<4, G><<<dim3(grid_for(c, most / 4, 256, c->light_blocks), nj), 256, 0, c->stream>>>(J, L);
+      else
+        k_vert_light<1, G><<<dim3(grid_for(c, most, 128, c->light_blocks), nj), 128, 0, c->stream>>>(J, L);
     });
+  };
+  if (nj > 4) light(VertJobs<MAX_GROUPS>());
+  else if (nj) light(VertJobs<4>());
   CK(cudaGetLastError());
   c->amb = amb;
   return 0;
