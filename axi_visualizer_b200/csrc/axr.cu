@@ -1807,6 +1807,7 @@ int batch_enqueue(axr_batch *b) {
   BatchParams B;
   B.views = b->d_views; B.nviews = (int)nv;
   B.groups_draw = b->d_gdraw; B.groups_shadow = b->d_gshadow; B.ngroups = BATCH_TABLE;
+  B.host_ctrs = b->mode == AXR_BATCH_PERSISTENT ? nullptr : b->h_ctrs;
   B.bar = b->d_bar; B.nblocks = (uint32_t)(b->grid + b->phantom); B.spin_limit = b->spin_limit;
   if (b->mode == AXR_BATCH_PERSISTENT) {
     void *args[] = {&B};
@@ -1833,6 +1834,7 @@ int batch_enqueue(axr_batch *b) {
     else kb_shade<false><<<sms * 4, 256, 0, s>>>(B);
     CK(cudaGetLastError());
   }
+  if (B.host_ctrs) return 0;
   for (size_t k = 0; k < nv; k++)
     CK(cudaMemcpyAsync(b->h_ctrs + k * CTR_N, b->buf[k].ctr, sizeof(uint32_t) * CTR_N, cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(b->h_bar, b->d_bar, sizeof(uint32_t) * BAR_WORDS, cudaMemcpyDeviceToHost, s));
@@ -2035,6 +2037,7 @@ int axr_batch_render(axr_batch *b, const int32_t *flags, const int32_t *alpha_in
   // the framebuffers are free once the last render's read-back has left them
   if (b->reads) CK(cudaStreamWaitEvent(c->stream, b->read_done, 0));
   b->reads = false;
+  if (b->mode != AXR_BATCH_PERSISTENT) memset(b->h_bar, 0, sizeof(uint32_t) * BAR_WORDS);   // no barriers, no stamps
   if (!b->exec) {
     if ((rc = batch_build_graph(b))) return rc;
   }

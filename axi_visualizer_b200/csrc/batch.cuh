@@ -38,6 +38,7 @@ struct BatchParams {
   int ngroups;
   uint32_t *bar;     // [0] arrivals, [1] generation, [2] barrier error, [3] blocks done,
                      // [4..15] six u64 globaltimer stamps: start, after phases 0-3, end
+  uint32_t *host_ctrs; // pinned host copies of the views' counters, written by the phased form's shade; null: none
   uint32_t nblocks;    // blocks the grid barrier waits for
   long spin_limit;     // polls before a waiting block gives up
 };
@@ -284,6 +285,13 @@ __global__ void __launch_bounds__(256, 4) kb_shade(BatchParams B) {
   __shared__ GroupDev sgd[BATCH_TABLE];
   __shared__ ShadeSmem<256> sm;
   for (int i = threadIdx.x; i < B.ngroups; i += blockDim.x) sgd[i] = B.groups_draw[i];
+  // the counters are final here; a copy a view took 3.5 us each of the copy
+  // engine, which the read-backs need (nine views: 391 -> 354 us a pass)
+  if (B.host_ctrs && blockIdx.x == 0)
+    for (int i = threadIdx.x; i < B.nviews * CTR_N; i += blockDim.x) {
+      const BatchView &V = B.views[i / CTR_N];
+      B.host_ctrs[i] = (V.kind == VIEW_DEPTH ? V.sp.ctr : V.dp.ctr)[i % CTR_N];
+    }
   __syncthreads();
   batch_shade<256, NRM>(B, sgd, sm);
 }
