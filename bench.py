@@ -36,32 +36,34 @@ W, H = 1920, 1080
 PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6650.0
 
-# From one `ncu --set full` capture of this frame's kernels (one launch per
-# kernel; the two cascades averaged for the shadow kernels, as the per-kernel
-# event times are): per launch, DRAM traffic (dram__bytes_read.sum +
-# dram__bytes_write.sum) and issued warp instructions (smsp__inst_issued.sum).
+# From one ncu capture of this frame's kernels: DRAM traffic per launch
+# (dram__bytes.sum; the two cascades averaged for the shadow kernels, as the
+# per-kernel event times are), and issued warp instructions of a frame's
+# launches (smsp__inst_issued.sum; the two cascades together).
 # A kernel whose code changed since its capture has no entry.  NCU_CAPTURE
 # names the committed summary of that capture, reported in the JSON line.
 NCU_CAPTURE = "profiles/ncu_kernels_1080p_1m.md"
 NCU_TRAFFIC = {
-    "k_raster_small": 33623552,
-    "k_raster_small_alpha": 13610240,
-    "k_shadow_raster": (48459520 + 52097024) // 2,
-    "k_shadow_raster_alpha": (10682368 + 4569856) // 2,
-    "k_shade": 35214336,
-    "k_raster_tiled_alpha": 8154624,
-    "k_shadow_setup": (37651968 + 37644800) // 2,
-    "k_setup": 55719424,
+    "k_raster_small": 32811008,
+    "k_raster_small_alpha": 13467648,
+    "k_shadow_raster": (46954496 + 50692096) // 2,
+    "k_shadow_raster_alpha": (10293248 + 4461568) // 2,
+    "k_shade": 30253056,
+    "k_raster_tiled": 10337280,
+    "k_raster_tiled_alpha": 8160256,
+    "k_shadow_setup": (37618944 + 37617920) // 2,
+    "k_setup": 54932224,
 }
 NCU_ISSUED = {
-    "k_raster_small": 144550486,
-    "k_raster_small_alpha": 101604329,
-    "k_shadow_raster": (224048127 + 130663712) // 2,
-    "k_shadow_raster_alpha": (48309342 + 21214830) // 2,
-    "k_shade": 95960306,
-    "k_raster_tiled_alpha": 47031883,
-    "k_shadow_setup": (16162323 + 16116092) // 2,
-    "k_setup": 16814245,
+    "k_raster_small": 83089658,
+    "k_raster_small_alpha": 69438194,
+    "k_shadow_raster": 144353943 + 83025235,
+    "k_shadow_raster_alpha": 34789834 + 12203377,
+    "k_shade": 78040365,
+    "k_raster_tiled": 20877990,
+    "k_raster_tiled_alpha": 29736853,
+    "k_shadow_setup": 14444480 + 14714699,
+    "k_setup": 14435226,
 }
 ISSUE_PER_SM_PER_CLK = 4     # warp instructions: one per scheduler (4 per SM) per cycle
 
@@ -174,9 +176,10 @@ def algorithmic_bytes(scene, q, shadow_q, visible_tris):
 
 
 def issue_of(kernel, avg_s, sms, sm_mhz):
-    """The instruction-issue roofline of a kernel: its issued warp
-    instructions per launch (ncu) / its CUDA-event launch time, against
-    sms x 4 schedulers x the SM clock sampled during the run."""
+    """The instruction-issue roofline of a kernel: the issued warp
+    instructions of a frame's launches of it (ncu) / `avg_s`, their CUDA-event
+    time in a frame, against sms x 4 schedulers x the SM clock sampled during
+    the run."""
     n = NCU_ISSUED.get(kernel)
     if n is None or not avg_s:
         return None
@@ -197,7 +200,7 @@ def roofline_of(kernel, ktimes, alg, hbm, peak_kind, steps, sms=148, sm_mhz=1965
     return {"bound": "hbm", "kernel": kernel, "achieved": achieved, "peak": hbm, "unit": "GB/s",
             "frac": achieved / hbm, "peak_source": peak_kind, "traffic": t,
             "traffic_capture": NCU_CAPTURE if t is not None else None, "algorithmic_bytes": a,
-            "avg_us": 1e6 * avg_s, "launches_per_frame": n / steps, "issue": issue_of(kernel, avg_s, sms, sm_mhz)}
+            "avg_us": 1e6 * avg_s, "launches_per_frame": n / steps, "issue": issue_of(kernel, avg_s * n / steps, sms, sm_mhz)}
 
 
 def frame_bytes(scene):
@@ -560,7 +563,7 @@ def vertex_section(R, view, hbm, frames=100, warmup=5):
             continue
         tot_ms, n = kt[name]
         avg_s = tot_ms / n / 1000.0
-        if nv is None:   # one launch per group: bytes of the average group
+        if nv is None:   # all lit vertices over a frame's launches
             nv = nv_all / (n / frames)
         gbs = per_v * nv / avg_s / 1e9
         out[name] = {"avg_us": avg_s * 1e6, "launches_per_frame": n / frames, "bytes_per_vertex": per_v,
@@ -573,9 +576,9 @@ def post_section(R, view, hbm, frames=50):
     CLDraw.blur) after every rendered frame: their kernels' CUDA-event times
     and HBM throughput.  ssao and dof: 16 algorithmic bytes a pixel each
     (depth and colour read, colour written; the gathered neighbours are
-    re-reads that stay in cache).  The bloom's four passes: 6 + 6 + 6 bytes
-    a half-resolution pixel and 12 a full-resolution one (colour read and
-    written by the final add)."""
+    re-reads that stay in cache).  The bloom's two launches: 6 + 6 bytes a
+    half-resolution pixel (the horizontal blur written and read) and 18 a
+    full-resolution one (colour read by both, written by the second)."""
     D = R.draw
     rnd = np.random.default_rng(44).random(48).astype(np.float32)
 
@@ -598,11 +601,11 @@ def post_section(R, view, hbm, frames=50):
         avg_s = tot_ms / n / 1000.0
         gbs = 16 * px / avg_s / 1e9
         out[name] = {"avg_us": avg_s * 1e6, "bytes_per_pixel": 16, "achieved_gbs": gbs, "frac_of_hbm": gbs / hbm}
-    names = ("k_bloom_bright", "k_bloom_blur_h", "k_bloom_blur_v", "k_bloom_add")
+    names = ("k_bloom_h", "k_bloom_v")
     if all(k in kt for k in names):
         half = (view.w // 2) * (view.h // 2)
         us = sum(1000 * kt[k][0] / kt[k][1] for k in names)
-        b = 18 * half + 12 * view.w * view.h
+        b = 12 * half + 18 * view.w * view.h
         out["bloom"] = {"avg_us": us, "passes_us": {k: 1000 * kt[k][0] / kt[k][1] for k in names},
                         "algorithmic_bytes": b, "achieved_gbs": b / us / 1e3, "frac_of_hbm": b / us / 1e3 / hbm}
     return out
@@ -921,7 +924,7 @@ def main():
     sms = torch.cuda.get_device_properties(local).multi_processor_count
     sm_mhz = clk["sm_mhz"] if clk else 1965.0
     for k, (ms, n) in ktimes.items():
-        iss = issue_of(k, ms / n / 1000.0, sms, sm_mhz)
+        iss = issue_of(k, ms / args.steps / 1000.0, sms, sm_mhz)
         if iss:
             per_kernel[k]["issue_frac"] = iss["frac"]
     dom = max(ktimes.items(), key=lambda kv: kv[1][0])[0]
