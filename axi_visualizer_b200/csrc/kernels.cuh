@@ -268,7 +268,7 @@ __device__ __forceinline__ V3 cross3(V3 a, V3 b) {
 }
 
 // The occlusion that a pixel's 16 samples add up to.  TAME: the sample's depth
-// is in [0.96, 2^14], its x and y below 2^35, ss in [1, 2^20] and w, h in
+// is in [0.46, 2^14], its x and y below 2^35, ss in [1, 2^20] and w, h in
 // [16, 2^20].  Then the shared reciprocal gives the IEEE quotients without a
 // look at each sample: a numerator below 2^-60, for which it need not, ends as
 // exactly w2 or h2 (>= 8) either way.  floor() of a coordinate, taken as unsigned,
@@ -334,8 +334,8 @@ __device__ __forceinline__ float ssao_samples(const float4 *T, const float *__re
 // 1080p frame.  Pixels beyond depth 6000 keep their colour (ao = 0) and take no
 // samples.  The two quotients by the sample depth share one reciprocal; the ranges
 // in which it gives the IEEE quotient are checked once a pixel, from its depth, its
-// normal and the block's table (ssao_samples), and by sample only where that fails:
-// nearer than 4, degenerate normals, unusual tables and scales.  Eight samples'
+// normal and the block's table (ssao_samples), and by sample only in warps where that
+// fails: nearer than 1.5, degenerate normals, unusual tables and scales.  Eight samples'
 // depth reads are in flight at a time.  Bound by instruction issue
 // (2.8 of 4 a cycle): 76 us of a 1080p frame; 91 with the range checks by sample and
 // four reads in flight, 133 with a table for every tile and samples one by one as
@@ -382,8 +382,10 @@ __global__ void __launch_bounds__(256) k_ssao(uint16_t *__restrict__ ro, uint16_
     V3 py = smul3(dy, V3{vx, quot_by_recip(-(fy + 1.f - h2), ss, yss), 1.f});
     V3 norm = fast_normalize(cross3(sub3(pos, px), sub3(pos, py)));   // rx * ry = 1
     V3 norm2 = smul3(2.f, norm);
-    // |norm| <= 1.005 and the table's checked lengths keep a sample within 3.04 of pos, so z >= 0.96
-    const bool tame = block_tame && d >= 4.f && dot3(norm, norm) <= 1.01f;
+    // A reflection about norm takes |sv|^2 to |sv|^2 + 4 dt^2 (|norm|^2 - 1): with the table's
+    // lengths a sample stays within 1.04 of pos, so its z is at least 0.46.  By warp, as one
+    // that ran both loops would take 161 us where 132 had done (near and far pixels mixed).
+    const bool tame = __all_sync(__activemask(), block_tame && d >= 1.5f && dot3(norm, norm) <= 1.01f);
     float ao = tame ? ssao_samples<true>(T, F, pos, norm, norm2, d, ss, w2, h2, w, h, (uint32_t)pix)
                     : ssao_samples<false>(T, F, pos, norm, norm2, d, ss, w2, h2, w, h, (uint32_t)pix);
     ao /= 16.f;

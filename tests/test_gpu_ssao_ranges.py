@@ -1,5 +1,5 @@
 """ssao at the edges of the ranges in which its samples need no checks of their
-own, against the oracle bit for bit: depths on both sides of 4, tables whose
+own, against the oracle bit for bit: depths on both sides of 1.5 and of 4, tables whose
 scaled lengths are below, at and beyond 1, scales inside and outside
 [1, 2^20], flat and noisy depths, heights that are
 no multiple of 16.
@@ -16,6 +16,10 @@ pytestmark = pytest.mark.gpu
 def depths(kind, w, h, rng):
     if kind == "near":                          # both sides of the bound, and values next to it
         return rng.choice(np.array([3.9999998, 4.0, 4.0000005, 1e-3, 0.5, 5.0], np.float32), (h, w))
+    if kind == "mixed":                         # both sides of 1.5 within a warp
+        return rng.choice(np.array([1.4999999, 1.5, 1.5000001, 1.6, 7.0, 0.2], np.float32), (h, w))
+    if kind == "close":                         # at and above 1.5 only
+        return rng.choice(np.array([1.5, 1.5000001, 1.75, 2.5], np.float32), (h, w))
     if kind == "flat":
         return np.full((h, w), 9.0, np.float32)
     if kind == "far":
@@ -24,7 +28,7 @@ def depths(kind, w, h, rng):
     return (4.0 + 0.02 * x + 0.03 * y + 0.3 * rng.random((h, w))).astype(np.float32)      # surfaces
 
 
-@pytest.mark.parametrize("kind", ["near", "flat", "far", "surface"])
+@pytest.mark.parametrize("kind", ["near", "mixed", "close", "flat", "far", "surface"])
 @pytest.mark.parametrize("table", [1.0, 1.1, 3.0])
 @pytest.mark.parametrize("scale", [None, 0.75, 1.0, 2.0 ** 20, 2.0 ** 21])
 def test_ssao_equals_oracle(kind, table, scale):
