@@ -349,7 +349,10 @@ __global__ void __launch_bounds__(TILE_THREADS, ALPHA ? 6 : 8) k_shadow_tiles(Sh
   __shared__ SpanQ<ALPHA> qs[TILE_THREADS / 32];
   __shared__ int smax[TILE_THREADS / 32][SUBS * SUBS];
   __shared__ uint32_t ready[TILE_THREADS / 32][64];
-  __shared__ uint32_t s_k;
+  // two words: a warp may still be about to read the claimed block number when
+  // thread 0 knows whether the tile has units left (with one word for both, warps
+  // of a block at times worked on different tiles)
+  __shared__ uint32_t s_k, s_done;
   for (int i = threadIdx.x; i < S.ngroups; i += blockDim.x) sg[i] = S.groups[i];
   __syncthreads();
   int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -375,13 +378,11 @@ __global__ void __launch_bounds__(TILE_THREADS, ALPHA ? 6 : 8) k_shadow_tiles(Sh
     uint32_t u0 = ALPHA ? S.tcur[2 * t] : S.toff[t];          // after binning: end of the opaque units
     uint32_t n = ALPHA ? S.tcur[2 * t + 1] - u0 : S.tcur[2 * t] - u0;
     uint32_t *claim = S.tclaim + 2 * t + (ALPHA ? 1 : 0);
-    // nothing left to claim (uniform: thread 0's read is shared after the barrier)
-    if (threadIdx.x == 0) s_k = n == 0 || *(volatile uint32_t *)claim >= n;
+    // nothing left to claim (uniform: thread 0's read is shared after the barrier;
+    // the next write of either word comes after a barrier that follows its reads)
+    if (threadIdx.x == 0) s_done = n == 0 || *(volatile uint32_t *)claim >= n;
     __syncthreads();
-    if (s_k) {
-      __syncthreads();
-      continue;
-    }
+    if (s_done) continue;
     int tx0 = (int)(t % (uint32_t)S.ntx) * STILE, ty0 = (int)(t / (uint32_t)S.ntx) * STILE;
     int tx1 = min(tx0 + STILE, dim) - 1, ty1 = min(ty0 + STILE, dim) - 1;
     int init[TEXELS_PER_THREAD];
