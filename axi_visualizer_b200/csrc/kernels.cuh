@@ -923,11 +923,17 @@ struct RowPair {
 };
 
 // Interpolants (1 / depth) of an item whose vertices' z pass this stay in
-// [2^-31, 2^59] on every row: they run from vertex to vertex and drift by at
-// most 2^-24 of the largest a row.  Differences of such z are 0 or at least
-// 2^-53, so slopes and pixels can take the reciprocal path.
-__device__ __forceinline__ bool z_safe(float z1, float z2, float z3) {
-  return z1 >= 0x1p-30f && z2 >= 0x1p-30f && z3 >= 0x1p-30f && z1 <= 0x1p58f && z2 <= 0x1p58f && z3 <= 0x1p58f;
+// [2^-32, 2^59] on every row, so pixels need no sign or range case, and
+// differences of such z are 0 or at least 2^-55, so slopes can take the
+// reciprocal path.  A walk of up to `rows` = y3 - y1 additions of a slope starts
+// at a vertex.  Each addition rounds by at most 2^-24 of the largest z, the slope
+// (difference, quotient or reciprocal, product) by 3 x 2^-24 of it over the whole
+// walk, and the split vertex's z by 4 x 2^-24, all but for factors 1 + rows 2^-24:
+// together (rows + 8) 2^-24 of the largest.  That moves the SMALLEST value too, so
+// it has to be at least twice that: the walk then stays above about half of it.
+__device__ __forceinline__ bool z_safe(float z1, float z2, float z3, float rows) {
+  const float hi = fmaxf(z1, fmaxf(z2, z3)), lo = fmaxf(0x1p-30f, hi * ((rows + 8.f) * 0x1p-23f));
+  return z1 >= lo && z2 >= lo && z3 >= lo && hi <= 0x1p58f;
 }
 
 // Writes a span's ends to `slot`: first pixel lo, edges cx1 / cx2 with 1/depth
@@ -1132,7 +1138,7 @@ __device__ __forceinline__ void vis_fill(const DrawParams &P, const GroupDev *sg
 template <bool ALPHA>
 struct SmallLane {
   int g;
-  bool safe;       // z_safe of its vertices
+  bool safe;       // z_safe of its vertices and rows
   uint32_t gtri;
   int x1, x2, x3, y1, y2, y3;
   float z1, z2, z3, x4, z4;
@@ -1261,7 +1267,7 @@ struct SmallLane {
     float yd = quot_fast((float)(y2 - y1), hgt, recip_rn(hgt));
     x4 = (float)x1 + yd * (float)(x3 - x1);
     z4 = z1 + yd * (z3 - z1);
-    safe = z_safe(z1, z2, z3);
+    safe = z_safe(z1, z2, z3, hgt);
     if (ALPHA) {
       uv4 = add2(a[0].uv, smul2(yd, sub2(a[2].uv, a[0].uv)));
       if (G.flags & F_MIP) mip_setup<false>(a, z, true, ix, iy, nullptr, nullptr, G.tex_size, G.mip_bias);
@@ -2535,7 +2541,7 @@ __device__ __noinline__ void shadow_serial(float *map, const GroupDev *sg, const
 
 template <bool ALPHA>
 struct ShadowLane {
-  bool safe;     // z_safe of its vertices
+  bool safe;     // z_safe of its vertices and rows
   int x1, x2, x3, y1, y2, y3, x4;
   float z1, z2, z3, z4, u1, u2, u3, u4, v1, v2, v3, v4;
   int half, cy, g;
@@ -2624,7 +2630,7 @@ struct ShadowLane {
   __device__ __forceinline__ void finish(const V2 uv[3]) {
     float hgt = (float)(y3 - y1);   // (0: one row, the split vertex is not used)
     float q = quot_fast((float)(y2 - y1), hgt, recip_rn(hgt));
-    safe = z_safe(z1, z2, z3);
+    safe = z_safe(z1, z2, z3, hgt);
     x4 = f2i((float)x1 + q * (float)(x3 - x1));
     z4 = z1 + q * (z3 - z1);
     if (ALPHA) {

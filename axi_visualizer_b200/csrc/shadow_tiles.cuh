@@ -247,7 +247,8 @@ __device__ __forceinline__ void refresh_smax(const int *tile, int *smax, int lan
 
 // True when record r's caster cannot lower any texel of the tile: the
 // smallest depth any of its pixels can store lies above the maxima of all
-// the sub-blocks its rows and (widened) columns touch.  Its 1/z
+// the sub-blocks its rows and (widened) columns touch.  Only for casters that
+// pass z_safe: another's walk may reach negative depths.  Its 1/z
 // interpolants stay below zmax (1 + (rows + 10) 2^-24) -- each of the at
 // most `rows` accumulated additions and the split vertex's z round by 2^-24
 // of their value -- and a pixel's 1/z below that times (1 + 2^-24)^3, so a
@@ -256,11 +257,12 @@ __device__ __forceinline__ void refresh_smax(const int *tile, int *smax, int lan
 __device__ __forceinline__ bool unit_hidden(const ShadowParams &S, uint32_t r, const int *smax, int tx0, int tx1,
                                             int ty0, int ty1) {
   uint4 a = S.rec[2 * (size_t)r], b = S.rec[2 * (size_t)r + 1];
-  float zmax = fmaxf(__uint_as_float(a.w), fmaxf(__uint_as_float(b.x), __uint_as_float(b.y)));
+  const float z1 = __uint_as_float(a.w), z2 = __uint_as_float(b.x), z3 = __uint_as_float(b.y);
+  float zmax = fmaxf(z1, fmaxf(z2, z3));
   int x[3] = {unpack_x(a.x), unpack_x(a.y), unpack_x(a.z)};
   int y1 = unpack_y(a.x), y3 = unpack_y(a.z);
   int rows = y3 - y1 + 1;
-  if (!(zmax >= 0x1p-60f) || !(zmax <= 0x1p60f) || rows > 65536) return false;
+  if (!z_safe(z1, z2, z3, (float)(y3 - y1))) return false;
   float rz;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rz) : "f"(zmax));
   float f = 1.0f - 0x1p-17f - (float)rows * 0x1p-22f;
