@@ -140,9 +140,11 @@ __device__ __forceinline__ float span_t(float n, float d, float y) {
 
 // RN(1 / v) for 2^-61 <= |v| < 2^62: the approximate reciprocal (within one
 // ulp) and one residual step, e = 1 - v r, r + r e, which Markstein's paper
-// shows to round correctly except perhaps for isolated mantissas; compared
-// with __frcp_rn over every mantissa, both signs and all these exponents it
-// has none.  Three instructions, no branch, against about ten.
+// shows to round correctly except perhaps for isolated mantissas.  Tried for
+// every mantissa and every start within one ulp, the one exception is 0x7fffff
+// (1.99999988) from 0.5; what the GPU starts from there gives the right result
+// (tests/test_gpu_reciprocal.py).  Three instructions, no branch, against about
+// ten.
 __device__ __forceinline__ float recip_rn(float v) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
