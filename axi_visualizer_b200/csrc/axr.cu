@@ -37,6 +37,7 @@ int fail(int code, const char *fmt, ...) {
   vsnprintf(buf, sizeof buf, fmt, ap);
   va_end(ap);
   g_err = buf;
+  if (code == AXR_ENOMEM) cudaGetLastError();   // else the next launch's check would report the refused allocation
   return code;
 }
 
@@ -229,6 +230,7 @@ int grow_units(axr_ctx *c, uint32_t need) {
   if (cap > 0x7fffffffull) cap = 0x7fffffffull;
   cudaFree(c->units);
   c->units = nullptr;
+  c->cap_units = 0;   // no room: every large triangle goes to the fallback kernel
   if (cudaMalloc(&c->units, sizeof(uint2) * cap) != cudaSuccess)
     return fail(AXR_ENOMEM, "tile-unit queue of %llu entries", (unsigned long long)cap);
   c->cap_units = (uint32_t)cap;

@@ -1,0 +1,72 @@
+"""Device allocations that fail, made to fail on the host.
+
+Each case runs in a child process with a shim in front of cudaMalloc that, when
+armed, lets a chosen later call ask the runtime for more memory than any GPU
+has.  The call that needed the memory reports it, and the handle draws the next
+frames exactly.
+"""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+static int left = -1;
+void shim_fail(int after) { left = after; }   /* the call number `after` from now; -1: none */
+int cudaMalloc(void **p, size_t n) {
+  static int (*real)(void **, size_t);
+  if (!real) real = (int (*)(void **, size_t))dlsym(dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), "cudaMalloc");
+  return real(p, left >= 0 && left-- == 0 ? (size_t)1 << 60 : n);
+}
+"""
+COMMON = """
+import ctypes, os, sys
+sys.path[:0] = sys.argv[1:4]
+import numpy as np, pytest
+import oracle as O
+from axi_visualizer_b200 import scenes as S
+from axi_visualizer_b200._lib import AxrError
+from axi_visualizer_b200.ops import SceneRenderer
+shim = ctypes.CDLL(os.environ["LD_PRELOAD"])
+sc = S.scene_small(seed=1, flags=S.MIP | S.SHADOW)
+views = [S.default_view(320, 240, pos=p) for p in ((3, 2, -8), (2, 3, -9), (1, 2, -7))]
+want = [O.render(sc, v)[0] for v in views]
+R = SceneRenderer(sc, 320, 240)
+
+def exact(k):
+    db = R.draw.getFrame()[3]
+    assert np.array_equal(db.view(np.uint32), want[k].db.view(np.uint32)), k
+"""
+CASES = {
+    # the tile-unit queue cannot grow after an overflow: later frames overflow
+    # again and are drawn by the fallback, until it can
+    "unit_queue": """
+R.frame(views[0])
+shim.shim_fail(0)
+with pytest.raises(AxrError, match="tile-unit queue"):
+    R.draw.sync()
+for k in (1, 2):
+    R.frame(views[k])
+    assert R.draw.lastStats()["n_units"] > 16
+    exact(k)
+""",
+}
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_failed_allocation(case, tmp_path):
+    src, so = tmp_path / "shim.c", tmp_path / "shim.so"
+    src.write_text(SHIM)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", str(so), str(src), "-ldl"], check=True)
+    root = os.path.dirname(HERE)
+    env = dict(os.environ, LD_PRELOAD=str(so), AXR_UNIT_QUEUE="16")
+    r = subprocess.run([sys.executable, "-c", COMMON + CASES[case], root, os.path.join(root, "oracle"), HERE], env=env,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
