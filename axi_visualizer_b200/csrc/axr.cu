@@ -1100,8 +1100,9 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
   // shading samples the cascades: wait for their last writers
   for (int k = 0; k < nshadow; k++)
     if ((rc = wait_writer(c, c->shadows[shadow_ids[k]]))) return rc;
-  // the shade writes the counters over those of the frame before last
-  if (c->pend[slot] && (rc = check_slot(c, slot, true))) return rc;
+  // the shade writes the counters over those of the frame before last; an
+  // error of that frame is reported when this one is complete
+  const int earlier = c->pend[slot] ? check_slot(c, slot, true) : 0;
   dim3 sb(256), sgd((c->w + 15) / 16, (c->h + 15) / 16);   // a 16x16 tile per block
   if (any_normal)
     launch(c, s, "k_shade", [&] { k_shade<true><<<sgd, sb, 0, s>>>(P); });
@@ -1114,7 +1115,7 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
   c->pend[slot] = true;
   c->last_slot = slot;
   c->last_kernels = nk;
-  return 0;
+  return earlier;
 }
 
 int axr_get_frame(axr_ctx *c, uint16_t *r, uint16_t *g, uint16_t *b, float *depth) {

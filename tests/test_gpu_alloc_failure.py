@@ -45,6 +45,25 @@ def exact(k):
     assert np.array_equal(db.view(np.uint32), want[k].db.view(np.uint32)), k
 """
 CASES = {
+    # the same while a frame is being drawn, which learns of the overflow of the
+    # frame before last: it reports that, and is complete all the same
+    "unit_queue_mid_frame": """
+import torch
+slow = torch.cuda.ExternalStream(R.draw.stream_ptr())
+with torch.cuda.stream(slow):
+    torch.cuda._sleep(200_000_000)    # both frames are still unfinished when the third is drawn
+R.frame(views[0])
+R.frame(views[1])
+R.shadow_pass()
+R.set_view(views[2])
+R.draw.clearZBuffer()
+shim.shim_fail(0)
+with pytest.raises(AxrError, match="tile-unit queue"):
+    R.draw.drawAll(R.shaders, shadowIds=[0, 1])
+exact(2)
+R.frame(views[1])
+exact(1)
+""",
     # the tile-unit queue cannot grow after an overflow: later frames overflow
     # again and are drawn by the fallback, until it can
     "unit_queue": """
