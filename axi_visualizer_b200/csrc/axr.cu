@@ -1353,8 +1353,11 @@ int axr_add_shadow_map(axr_ctx *c, int i, int size, float scale, float amb) {
     size_t nt = (size_t)s.ntx * s.ntx;
     if (cudaMalloc(&s.map, sizeof(float) * (size_t)size * size) != cudaSuccess ||
         cudaMalloc(&s.ctr, sizeof(uint32_t) * (2 * CTR_N + 4 * nt)) != cudaSuccess ||
-        cudaMalloc(&s.tiles, sizeof(uint32_t) * (5 * nt + 1)) != cudaSuccess)
+        cudaMalloc(&s.tiles, sizeof(uint32_t) * (5 * nt + 1)) != cudaSuccess) {
+      cudaFree(s.map); cudaFree(s.ctr);
+      s.map = nullptr; s.ctr = s.tiles = nullptr;   // the map does not exist
       return fail(AXR_ENOMEM, "shadow map %dx%d", size, size);
+    }
     s.clean[0] = s.clean[1] = false;
   }
   s.dim = size;
@@ -1979,6 +1982,10 @@ int axr_batch_render(axr_batch *b, const int32_t *flags, const int32_t *alpha_in
                                                     c->groups.size());
   if ((uint32_t)std::max(c->total_tris, 1) > b->cap_list) return fail(AXR_ESTATE, "groups were added after the batch was created");
   if ((rc = batch_settle(b))) return rc;       // the previous render has left the pinned tables
+  for (auto &v : b->desc)
+    for (int j = 0; j < v.ncascades; j++)
+      if (v.cascades[j] < 0 && !c->shadows[-1 - v.cascades[j]].map)
+        return fail(AXR_ESTATE, "shadow map %d does not exist", -1 - v.cascades[j]);
   for (auto &v : b->desc) {
     if (v.kind != AXR_VIEW_SHADED || v.ncascades > 0 || !flags) continue;
     int gf, gn;

@@ -45,6 +45,18 @@ def exact(k):
     assert np.array_equal(db.view(np.uint32), want[k].db.view(np.uint32)), k
 """
 CASES = {
+    # the tile-unit queue cannot grow after an overflow: later frames overflow
+    # again and are drawn by the fallback, until it can
+    "unit_queue": """
+R.frame(views[0])
+shim.shim_fail(0)
+with pytest.raises(AxrError, match="tile-unit queue"):
+    R.draw.sync()
+for k in (1, 2):
+    R.frame(views[k])
+    assert R.draw.lastStats()["n_units"] > 16
+    exact(k)
+""",
     # the same while a frame is being drawn, which learns of the overflow of the
     # frame before last: it reports that, and is complete all the same
     "unit_queue_mid_frame": """
@@ -64,17 +76,25 @@ exact(2)
 R.frame(views[1])
 exact(1)
 """,
-    # the tile-unit queue cannot grow after an overflow: later frames overflow
-    # again and are drawn by the fallback, until it can
-    "unit_queue": """
-R.frame(views[0])
-shim.shim_fail(0)
-with pytest.raises(AxrError, match="tile-unit queue"):
-    R.draw.sync()
-for k in (1, 2):
+    # a shadow map without its counters does not exist, and can be made later
+    "shadow_map": """
+from axi_visualizer_b200.batch import Batch, shaded
+cam = sc.shadows[0]
+flags = [g.flags for g in sc.groups]
+B = Batch(R.draw, [shaded(views[0], (-1, -2))])
+shim.shim_fail(1)
+with pytest.raises(AxrError, match="shadow map 96x96"):
+    R.draw.addShadowMap(0, 96, cam.scale, 0.2)
+with pytest.raises(AxrError, match="does not exist"):
+    R.draw.shadowMap(0, [g.cast for g in sc.groups], R.shaders, sc.bias)
+with pytest.raises(AxrError, match="does not exist"):
+    B.render(flags)
+R.draw.addShadowMap(0, cam.dim, cam.scale, 0.2)
+for k in range(3):
     R.frame(views[k])
-    assert R.draw.lastStats()["n_units"] > 16
     exact(k)
+B.render(flags, [g.alpha_index for g in sc.groups])
+assert np.array_equal(B.frame(0)[3].view(np.uint32), want[0].db.view(np.uint32))
 """,
 }
 
