@@ -732,9 +732,13 @@ int axr_add_texture_group(axr_ctx *c, const float *xyz, const float *uv, const f
     return rc;
   if (cudaMalloc(&G.li, sizeof(float) * std::max<size_t>(nv * 3, 1)) != cudaSuccess) return fail(AXR_ENOMEM, "LI buffer");
   CK(cudaMemsetAsync(G.li, 0, sizeof(float) * nv * 3, c->stream));
-  c->groups.push_back(G);
   c->total_tris += ntris;
-  if ((rc = ensure_lists(c))) return rc;
+  if ((rc = ensure_lists(c))) {   // the group is not added
+    c->total_tris -= ntris;
+    cudaFree(G.xyz); cudaFree(G.vn); cudaFree(G.uv); cudaFree(G.tex); cudaFree(G.li);
+    return rc;
+  }
+  c->groups.push_back(G);
   CK(cudaStreamSynchronize(c->stream));   // host arrays are borrowed only for the call
   if (out_id) *out_id = (int)c->groups.size() - 1;
   return 0;
@@ -1023,7 +1027,7 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
   if (rc) return rc;
   if (ngroups != (int)c->groups.size()) return fail(AXR_EINVAL, "drawAll with %d groups, handle has %zu", ngroups, c->groups.size());
   if (nshadow < 0 || nshadow > 2) return fail(AXR_EINVAL, "at most two shadow cascades");
-  if ((rc = settle_next(c))) return rc;
+  if ((rc = settle_next(c)) || (rc = ensure_lists(c))) return rc;   // (lists that could not grow were freed)
   DrawParams P;
   memset(&P, 0, sizeof P);
   bool any_shadow = false, any_alpha = false, any_normal = false;
@@ -1399,6 +1403,7 @@ int axr_shadow_map(axr_ctx *c, int i, const uint8_t *cast, const int32_t *flags,
   if (i < 0 || i >= MAX_SHADOWS || !c->shadows[i].map) return fail(AXR_ESTATE, "shadow map %d does not exist", i);
   if (ngroups != (int)c->groups.size() || !cast) return fail(AXR_EINVAL, "shadowMap arguments");
   if (!c->tpend.empty() && (rc = settle(c))) return rc;   // (with per-kernel timing)
+  if ((rc = ensure_lists(c))) return rc;
   // alpha casters use the alpha mask's own side as lenT (drawminalpha.c:86-96)
   std::vector<int32_t> fl(ngroups, 0);
   for (int g = 0; g < ngroups; g++) fl[g] = flags ? (flags[g] & (F_ALPHA | F_MIP)) : 0;

@@ -96,6 +96,18 @@ for k in range(3):
 B.render(flags, [g.alpha_index for g in sc.groups])
 assert np.array_equal(B.frame(0)[3].view(np.uint32), want[0].db.view(np.uint32))
 """,
+    # the triangle lists cannot grow for another group: it is not added, and the
+    # others are drawn as before
+    "triangle_lists": """
+g = sc.groups[0]
+planes = sc.groups[2].tex
+shim.shim_fail(5)                     # after the group's five arrays
+with pytest.raises(AxrError, match="triangle lists"):
+    R.draw.addTextureGroup(np.concatenate([g.xyz] * 40), np.concatenate([g.uv] * 40), np.concatenate([g.vn] * 40), *planes)
+for k in range(3):
+    R.frame(views[k])
+    exact(k)
+""",
 }
 
 
