@@ -183,7 +183,7 @@ struct axr_ctx {
   uint16_t *post[3] = {nullptr, nullptr, nullptr};   // dof's gather target (SSRO/SSGO/SSBO)
   uint16_t *bloom = nullptr;                           // the bloom's 3 half-resolution planes
   int ssao_blocks = 4;                       // resident 256-thread blocks of k_ssao per SM
-  int light_blocks = 4;                      // resident 256-thread blocks of k_vert_light per SM
+  int light_blocks[2] = {12, 4};             // resident blocks of k_vert_light<1> and <4> per SM
   // launch accounting and optional per-kernel CUDA-event timing
   int64_t launches = 0;
   int min_chunk = 0;                         // rows per work item set by axr_set_tuning (0: by the scene's size)
@@ -613,8 +613,9 @@ int axr_create(int w, int h, int device, axr_ctx **out) {
       cudaEventCreateWithFlags(&c->ev_lights, cudaEventDisableTiming) != cudaSuccess) {
     rc = fail(AXR_ENOMEM, "framebuffers for %dx%d", w, h);
   }
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->light_blocks, k_vert_light<4, 4>, 256, 0);
-  if (c->light_blocks < 1) c->light_blocks = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->light_blocks[0], k_vert_light<1, 4>, light_threads(1), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->light_blocks[1], k_vert_light<4, 4>, light_threads(4), 0);
+  for (int &b : c->light_blocks) b = std::max(b, 1);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->ssao_blocks, k_ssao, 256, 0);
   if (c->ssao_blocks < 1) c->ssao_blocks = 1;
   // initial tile-unit queue (grows after an overflow); AXR_UNIT_QUEUE overrides
@@ -804,20 +805,23 @@ int axr_vert_light(axr_ctx *c, const uint8_t *mask, int ngroups, const float *di
   L.nd = ndirs; L.np = npoints; L.ns = nspots; L.amb = amb;
   VertJob jobs[MAX_GROUPS];
   int nj = 0, most = 0;
+  int64_t all = 0;
   for (int g = 0; g < ngroups; g++) {
     const Group &G = c->groups[g];
     if ((mask && !mask[g]) || !G.ntris) continue;
     jobs[nj++] = {G.xyz, G.vn, G.li, G.ntris * 3};
     most = std::max(most, G.ntris * 3);
+    all += G.ntris * 3;
   }
   auto light = [&](auto J) {
     constexpr int G = sizeof J.g / sizeof J.g[0];
     std::copy(jobs, jobs + nj, J.g);
     launch(c, c->stream, "k_vert_light", [&] {
-      if (most >= c->sms * 1024)
-        k_vert_light<4, G><<<dim3(grid_for(c, most / 4, 256, c->light_blocks), nj), 256, 0, c->stream>>>(J, L);
+      constexpr int T1 = light_threads(1), T4 = light_threads(4);
+      if (all >= c->sms * 2048)
+        k_vert_light<4, G><<<dim3(grid_for(c, most / 4, T4, c->light_blocks[1]), nj), T4, 0, c->stream>>>(J, L);
       else
-        k_vert_light<1, G><<<dim3(grid_for(c, most, 128, c->light_blocks), nj), 128, 0, c->stream>>>(J, L);
+        k_vert_light<1, G><<<dim3(grid_for(c, most, T1, c->light_blocks[0]), nj), T1, 0, c->stream>>>(J, L);
     });
   };
   if (nj > 4) light(VertJobs<MAX_GROUPS>());

@@ -740,23 +740,33 @@ __device__ __forceinline__ void vert_light_n(const VertLights &L, const V3 x[N],
 struct VertJob { const float *xyz, *vn; float *li; int nv; };
 template <int G>
 struct VertJobs { VertJob g[G]; };
-// N = 1, one vertex a thread, for groups that would not fill the GPU with four:
-// the time is then one thread's chain over the lights (3,840 vertices under
-// 2 + 2 + 1 lights, with events: 9.4 us, 11.4 with four a thread).  G: groups in
-// the argument; a short one costs a small call less.
+// N = 1, one vertex a thread, for calls that would not fill the GPU with four:
+// the time is then one thread's chain over the lights.  40 registers, as the quads'
+// code is not compiled in: 1,536 threads an SM.  One group under the same lights,
+// with events, one a thread and four: 3,840 vertices 11.8 and 17.4 us, 160,000
+// 14.9 and 19.9, 300,000 18.2 and 19.1, 450,000 22.8 and 20.8; 16 groups of
+// 50,000 33.3 and 33.2, 64 of 50,000 109 and 97.  So the line is at 2,048 vertices an
+// SM, of all groups of the call (axr_vert_light).  G: groups in the argument; a
+// short one costs a small call less.
+constexpr int light_threads(int n) { return n == 4 ? 256 : 128; }
 template <int N, int G>
-__global__ void k_vert_light(const __grid_constant__ VertJobs<G> J, VertLights L) {
+__global__ void __launch_bounds__(light_threads(N), N == 4 ? 4 : 12)
+    k_vert_light(const __grid_constant__ VertJobs<G> J, VertLights L) {
   const VertJob &g = J.g[blockIdx.y];
   const bool pos = L.np + L.ns > 0;
-  const int nq = N == 4 ? g.nv >> 2 : 0;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-    V3 x[4] = {}, n[4], light[4];
-    if (pos) quad_ld(g.xyz, q, x);
-    quad_ld(g.vn, q, n);
-    vert_light_n<4>(L, x, n, light);
-    quad_st(g.li, q, light);
+  const uint32_t nv = g.nv, first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  uint32_t done = 0;
+  if constexpr (N == 4) {
+    for (int q = first; q < (int)(nv >> 2); q += step) {
+      V3 x[4] = {}, n[4], light[4];
+      if (pos) quad_ld(g.xyz, q, x);
+      quad_ld(g.vn, q, n);
+      vert_light_n<4>(L, x, n, light);
+      quad_st(g.li, q, light);
+    }
+    done = nv & ~3u;
   }
-  for (int v = (nq << 2) + blockIdx.x * blockDim.x + threadIdx.x; v < g.nv; v += gridDim.x * blockDim.x) {
+  for (uint32_t v = done + first; v < nv; v += step) {
     V3 x[1] = {}, n[1] = {ld3(g.vn + 3 * (size_t)v)}, light[1];
     if (pos) x[0] = ld3(g.xyz + 3 * (size_t)v);
     vert_light_n<1>(L, x, n, light);
