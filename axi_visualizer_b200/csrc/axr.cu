@@ -1201,7 +1201,7 @@ int axr_read_frame_rgb8_async(axr_ctx *c, float exposure, uint8_t *rgb, int64_t 
   }
   cudaStream_t s = c->stream;
   launch(c, s, "k_pack_rgb8", [&] {
-    k_pack_rgb8<<<grid_for(c, (long)n / 4, 256, 8), 256, 0, s>>>(c->ro, c->go, c->bo, (int)n, exposure, sl.stage);
+    k_pack_rgb8<<<grid_for(c, (long)n / 2, 256, 8), 256, 0, s>>>(c->ro, c->go, c->bo, (int)n, exposure, sl.stage);
   });
   CK(cudaGetLastError());
   CK(cudaEventRecord(sl.staged, s));
@@ -1274,7 +1274,7 @@ int axr_gamma(axr_ctx *c, float ex) {
   int rc = check_ctx(c);
   if (rc) return rc;
   long n = (long)c->w * c->h;
-  launch(c, c->stream, "k_gamma", [&] { k_gamma<<<grid_for(c, n / 8, 256, 8), 256, 0, c->stream>>>(c->ro, c->go, c->bo, (int)n, ex); });
+  launch(c, c->stream, "k_gamma", [&] { k_gamma<<<grid_for(c, n / 2, 256, 8), 256, 0, c->stream>>>(c->ro, c->go, c->bo, (int)n, ex); });
   CK(cudaGetLastError());
   return 0;
 }

@@ -212,43 +212,40 @@ __device__ __forceinline__ void gamma_px(uint32_t r, uint32_t g, uint32_t b, flo
   bo = trunc16(fminf(255.f, jz));
 }
 
-// Eight pixels a thread (the width is a multiple of 16): one 16-byte load and
-// store a plane.  Bound by issue and the square roots:
-// 15 us of a 1080p frame, 17 with two bytes a load and three divisions a pixel.
+// Two pixels a thread (the width is a multiple of 16): one 4-byte load and store
+// a plane.  Bound by issue and the square roots.  With events, one pixel and three
+// divisions a pixel, eight pixels, two: 64x64 6.5, 8.6, 6.6 us; 1280x720 10.7,
+// 10.7, 8.9; 1920x1080 14.8, 14.8, 12.9; 3840x2160 39.4, 37.2, 33.2.  More pixels a
+// thread are a longer chain for small frames, and save nothing in large ones.
 __global__ void __launch_bounds__(256, 8) k_gamma(uint16_t *r, uint16_t *g, uint16_t *b, int n, float exposure) {
   const float e8 = 8 * exposure;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / 8; i += gridDim.x * blockDim.x) {
-    uint4 R = reinterpret_cast<uint4 *>(r)[i], G = reinterpret_cast<uint4 *>(g)[i], B = reinterpret_cast<uint4 *>(b)[i];
-    uint32_t *pr = &R.x, *pg = &G.x, *pb = &B.x;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      uint32_t x0, y0, z0, x1, y1, z1;
-      gamma_px(pr[k] & 0xffffu, pg[k] & 0xffffu, pb[k] & 0xffffu, e8, x0, y0, z0);
-      gamma_px(pr[k] >> 16, pg[k] >> 16, pb[k] >> 16, e8, x1, y1, z1);
-      pr[k] = x0 | x1 << 16; pg[k] = y0 | y1 << 16; pb[k] = z0 | z1 << 16;
-    }
-    reinterpret_cast<uint4 *>(r)[i] = R; reinterpret_cast<uint4 *>(g)[i] = G; reinterpret_cast<uint4 *>(b)[i] = B;
+  uint32_t *pr = reinterpret_cast<uint32_t *>(r), *pg = reinterpret_cast<uint32_t *>(g), *pb = reinterpret_cast<uint32_t *>(b);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / 2; i += gridDim.x * blockDim.x) {
+    const uint32_t R = pr[i], G = pg[i], B = pb[i];
+    uint32_t x0, y0, z0, x1, y1, z1;
+    gamma_px(R & 0xffffu, G & 0xffffu, B & 0xffffu, e8, x0, y0, z0);
+    gamma_px(R >> 16, G >> 16, B >> 16, e8, x1, y1, z1);
+    pr[i] = x0 | x1 << 16; pg[i] = y0 | y1 << 16; pb[i] = z0 | z1 << 16;
   }
 }
 
 // Post/gamma.c's mapping packed as interleaved 8-bit RGB for display (the
-// planes are left as they are): 3 bytes per pixel instead of 6 + 4.  Four
-// pixels a thread: three whole words out.
+// planes are left as they are): 3 bytes per pixel instead of 6 + 4.  Two pixels
+// a thread, three half-words out: 128x96 8.3 us (one pixel 8.1, four 8.9),
+// 1920x1080 17.7 (18.4, 18.0; with three divisions a pixel 19.2).
 __global__ void k_pack_rgb8(const uint16_t *__restrict__ r, const uint16_t *__restrict__ g,
                             const uint16_t *__restrict__ b, int n, float exposure, uint8_t *__restrict__ out) {
   const float e8 = 8 * exposure;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / 4; i += gridDim.x * blockDim.x) {
-    uint2 R = reinterpret_cast<const uint2 *>(r)[i], G = reinterpret_cast<const uint2 *>(g)[i],
-          B = reinterpret_cast<const uint2 *>(b)[i];
-    uint32_t x[4], y[4], z[4];
-    gamma_px(R.x & 0xffffu, G.x & 0xffffu, B.x & 0xffffu, e8, x[0], y[0], z[0]);
-    gamma_px(R.x >> 16, G.x >> 16, B.x >> 16, e8, x[1], y[1], z[1]);
-    gamma_px(R.y & 0xffffu, G.y & 0xffffu, B.y & 0xffffu, e8, x[2], y[2], z[2]);
-    gamma_px(R.y >> 16, G.y >> 16, B.y >> 16, e8, x[3], y[3], z[3]);
-    uint32_t *o = reinterpret_cast<uint32_t *>(out) + 3 * (size_t)i;
-    o[0] = x[0] | y[0] << 8 | z[0] << 16 | x[1] << 24;
-    o[1] = y[1] | z[1] << 8 | x[2] << 16 | y[2] << 24;
-    o[2] = z[2] | x[3] << 8 | y[3] << 16 | z[3] << 24;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n / 2; i += gridDim.x * blockDim.x) {
+    const uint32_t R = reinterpret_cast<const uint32_t *>(r)[i], G = reinterpret_cast<const uint32_t *>(g)[i],
+                   B = reinterpret_cast<const uint32_t *>(b)[i];
+    uint32_t x0, y0, z0, x1, y1, z1;
+    gamma_px(R & 0xffffu, G & 0xffffu, B & 0xffffu, e8, x0, y0, z0);
+    gamma_px(R >> 16, G >> 16, B >> 16, e8, x1, y1, z1);
+    uint16_t *o = reinterpret_cast<uint16_t *>(out) + 3 * (size_t)i;
+    o[0] = (uint16_t)(x0 | y0 << 8);
+    o[1] = (uint16_t)(z0 | x1 << 8);
+    o[2] = (uint16_t)(y1 | z1 << 8);
   }
 }
 
