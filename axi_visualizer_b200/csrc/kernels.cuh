@@ -103,12 +103,16 @@ __device__ __forceinline__ int small_rows(int y1, int y3) { return y3 - y1 + 2; 
 // any number (alpha-tested queues, casters) or always 32 (opaque): 640x480 /
 // 24k triangles alone 225 -> 183 us, 88 -> 77 us among other frames; 720p /
 // 300k 336 -> 316 and 1080p / 1.04M 886 -> 869 among others (alone 970 -> 990).
+// A queue of fewer items than warps leaves most of the GPU idle whatever the claim,
+// so `least` falls with n / nw there (376 triangles at 320x192, the view alone, 135
+// -> 120 us; 1,552 at 1280x720 204 -> 189).
 // k = 0: always 32 -- the batched launches, whose warps move on to the
 // next view's queue when one runs dry, so no warp idles.
 __device__ __forceinline__ uint32_t claim_size(uint32_t n, uint32_t k, uint32_t least) {
   if (k == 0) return 32u;
   uint32_t nw = gridDim.x * (blockDim.x >> 5) * k;
   uint32_t per = (n + nw - 1) / nw;
+  if (n < nw) least = max((least * n + nw - 1) / nw, 1u);
   return per < least ? least : (per > 32u ? 32u : per);
 }
 constexpr uint32_t CLAIM_LEAST = 8;   // of the rasterizers
@@ -2786,7 +2790,13 @@ __device__ __forceinline__ void shadow_warp_loop(const ShadowParams &S, const Gr
   uint32_t n = chunked ? S.ctr[ALPHA ? CTR_SH_ITEMS_A : CTR_SH_ITEMS] : S.ctr[ctr_list];
   uint32_t cap_items = S.cap_list * MAX_CHUNKS;
   int dim = S.sh.dim;
-  const uint32_t per = claim_size(n, (uint32_t)S.claim_k, CLAIM_LEAST);
+  // A caster's item may be as wide as the map, and a claim of several such items is
+  // one warp's chain.  The more texels the map has an item, the wider they can be:
+  // fewer than 8 a claim from 1,024 texels an item.  With 8 throughout, 376
+  // triangles over 4096 and 2048 cascades (4K) took 1452 us a frame, now 496; 816
+  // 640, now 486; 176 over 1024 and 512 (720p) 273, now 102; 41,800 there 156, now 157.
+  const uint32_t least = min(max(n / max((uint32_t)(dim * dim) / 8192u, 1u), 1u), CLAIM_LEAST);
+  const uint32_t per = claim_size(n, (uint32_t)S.claim_k, least);
   while (true) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(&S.ctr[ctr_work], per);
