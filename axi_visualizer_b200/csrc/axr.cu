@@ -124,6 +124,12 @@ constexpr int SIDE_STREAM_TRIS = 8192;
 // 2019; 1080p / 1.04M 813, 798, 790; 720p / 300k 292, 287, 285, but alone 382,
 // 382, 397, and the normal-mapped 1296x713 view 157, 157, 165.
 constexpr int LONG_ITEM = 20, LONG_ITEM_TRIS = 700000;
+// From 1.5 drawn triangles a pixel the shade has the set-up by pair of row and
+// winner (its tiles may then hold up to 256 winners of a row each).  That code
+// costs the others registers: with it everywhere a view of 2,512 triangles at 4K
+// takes 563 us, not 551, 1.04M at 1080p 473 and 469; the figures of dense views
+// stand beside shade_tile.
+bool dense_view(int64_t tris, int w, int h) { return 2 * tris >= 3 * (int64_t)w * h; }
 constexpr int MAX_SHADOWS = 16;
 // 3 * ntris + 3 stays an int: the vertex kernels round v_end up to a quad
 constexpr int MAX_GROUP_TRIS = (INT_MAX - 3) / 3;
@@ -1040,7 +1046,9 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
   DrawParams P;
   memset(&P, 0, sizeof P);
   bool any_shadow = false, any_alpha = false, any_normal = false;
+  int64_t drawn = 0;
   for (int g = 0; g < ngroups; g++) {
+    if (!mask || !mask[g]) drawn += c->groups[g].ntris;
     if ((!mask || !mask[g]) && flags && (flags[g] & F_SHADOW)) any_shadow = true;
     if ((!mask || !mask[g]) && flags && (flags[g] & F_ALPHA)) any_alpha = true;
     if ((!mask || !mask[g]) && flags && (flags[g] & F_NORMAL)) any_normal = true;
@@ -1117,10 +1125,13 @@ int axr_draw_all(axr_ctx *c, const int32_t *flags, const int32_t *alpha_index, c
   // error of that frame is reported when this one is complete
   const int earlier = c->pend[slot] ? check_slot(c, slot, true) : 0;
   dim3 sb(256), sgd((c->w + 15) / 16, (c->h + 15) / 16);   // a 16x16 tile per block
-  if (any_normal)
-    launch(c, s, "k_shade", [&] { k_shade<true><<<sgd, sb, 0, s>>>(P); });
-  else
-    launch(c, s, "k_shade", [&] { k_shade<false><<<sgd, sb, 0, s>>>(P); });
+  launch(c, s, "k_shade", [&] {
+    const bool dense = dense_view(drawn, c->w, c->h);
+    if (any_normal && dense) k_shade<true, true><<<sgd, sb, 0, s>>>(P);
+    else if (any_normal) k_shade<true, false><<<sgd, sb, 0, s>>>(P);
+    else if (dense) k_shade<false, true><<<sgd, sb, 0, s>>>(P);
+    else k_shade<false, false><<<sgd, sb, 0, s>>>(P);
+  });
   nk++;
   CK(cudaGetLastError());
   CK(cudaEventRecord(c->ev_ctr[slot], s));
@@ -1660,7 +1671,8 @@ struct axr_batch {
   cudaStream_t side = nullptr;  // phased form: the alpha-tested branch
   cudaEvent_t done = nullptr, read_done = nullptr, ev_fork = nullptr, ev_coarse = nullptr, ev_join = nullptr;
   int mode = AXR_BATCH_PERSISTENT;
-  bool shade_nrm = true;   // the shade variant launched (and captured): with the normal-mapped core
+  // the shade variant launched (and captured): with the normal-mapped core, with the set-up by pair
+  bool shade_nrm = true, shade_dense = false;
   int phantom = 0;                  // fault injection: barrier waits for blocks never launched
   long spin_limit = BARRIER_SPIN_LIMIT;
   bool graph = false, pending = false, reads = false;
@@ -1851,8 +1863,10 @@ int batch_enqueue(axr_batch *b) {
     kb_tiled<false><<<sms * 8, 128, 0, s>>>(B);
     CK(cudaStreamWaitEvent(s, b->ev_join, 0));
     kb_fallback<<<sms * 4, 128, 0, s>>>(B);
-    if (b->shade_nrm) kb_shade<true><<<sms * 4, 256, 0, s>>>(B);
-    else kb_shade<false><<<sms * 4, 256, 0, s>>>(B);
+    if (b->shade_nrm && b->shade_dense) kb_shade<true, true><<<sms * 4, 256, 0, s>>>(B);
+    else if (b->shade_nrm) kb_shade<true, false><<<sms * 4, 256, 0, s>>>(B);
+    else if (b->shade_dense) kb_shade<false, true><<<sms * 4, 256, 0, s>>>(B);
+    else kb_shade<false, false><<<sms * 4, 256, 0, s>>>(B);
     CK(cudaGetLastError());
   }
   if (B.host_ctrs) return 0;
@@ -2042,17 +2056,24 @@ int axr_batch_render(axr_batch *b, const int32_t *flags, const int32_t *alpha_in
     b->goff[k] = seg_off[j];
   }
   batch_fill_views(b);
-  // the shade variant: with the normal-mapped core only when a shaded view
-  // draws such a material (a change rebuilds the captured graph)
-  bool nrm = false;
+  // the shade variant: with the normal-mapped core only when a shaded view draws
+  // such a material, with the set-up by pair once one was dense (a change
+  // rebuilds the captured graph)
+  bool nrm = false, dense = b->shade_dense;
   for (auto &v : b->desc) {
     if (v.kind != AXR_VIEW_SHADED || !flags) continue;
     int gf, gn;
     view_range(c, v, gf, gn);
-    for (int g = gf; g < gf + gn; g++) nrm = nrm || (flags[g] & F_NORMAL) != 0;
+    int64_t tris = 0;
+    for (int g = gf; g < gf + gn; g++) {
+      nrm = nrm || (flags[g] & F_NORMAL) != 0;
+      tris += c->groups[g].ntris;
+    }
+    dense = dense || dense_view(tris, v.w, v.h);
   }
-  if (nrm != b->shade_nrm) {
+  if (nrm != b->shade_nrm || dense != b->shade_dense) {
     b->shade_nrm = nrm;
+    b->shade_dense = dense;
     if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
   }
   // shaded views sampling the handle's own shadow maps wait for their writers

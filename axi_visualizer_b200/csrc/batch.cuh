@@ -171,22 +171,22 @@ __device__ __forceinline__ void batch_raster(const BatchParams &B, const GroupDe
 // phase 4: shading, tile by tile (16 x NT/16 pixels per block and tile);
 // NRM: some view draws a normal-mapped material (else the shade without
 // that core, which runs with fewer registers)
-template <int NT, bool NRM>
-__device__ __forceinline__ void batch_shade(const BatchParams &B, const GroupDev *sgd, ShadeSmem<NT> &sm) {
+template <int NT, bool NRM, bool DENSE>
+__device__ __forceinline__ void batch_shade(const BatchParams &B, const GroupDev *sgd, ShadeSmem<NT, NRM, DENSE> &sm) {
   constexpr int TH = NT / 16;
   for (int v = 0; v < B.nviews; v++) {
     const BatchView &V = B.views[v];
     if (V.kind != VIEW_SHADED) continue;
     int tw = (V.w + 15) / 16, th = (V.h + TH - 1) / TH;
     for (int t = blockIdx.x; t < tw * th; t += gridDim.x)
-      shade_tile<NT, NRM>(V.dp, sgd + V.goff, (t % tw) * 16, (t / tw) * TH, sm);
+      shade_tile<NT, NRM, DENSE>(V.dp, sgd + V.goff, (t % tw) * 16, (t / tw) * TH, sm);
   }
 }
 
 template <bool NRM>
 __global__ void __launch_bounds__(128, 4) k_batch(BatchParams B) {
   __shared__ GroupDev sgd[BATCH_TABLE], sgs[BATCH_TABLE];
-  __shared__ union U { WarpQueue wq[4]; ShadeSmem<128> sh; } u;   // phases 2-3 / phase 4
+  __shared__ union U { WarpQueue wq[4]; ShadeSmem<128, NRM, true> sh; } u;   // phases 2-3 / phase 4
   WarpQueue *wq = u.wq;
   load_tables(B, sgd, sgs);
   stamp(B.bar, 0);
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(128, 4) k_batch(BatchParams B) {
   if (!grid_sync(B.bar, B.nblocks, B.spin_limit)) return;
   stamp(B.bar, 4);
 
-  batch_shade<128, NRM>(B, sgd, u.sh);
+  batch_shade<128, NRM, true>(B, sgd, u.sh);
   // the last block to finish stamps the end
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -280,10 +280,10 @@ __global__ void __launch_bounds__(128) kb_fallback(BatchParams B) {
   }
 }
 
-template <bool NRM>
+template <bool NRM, bool DENSE>
 __global__ void __launch_bounds__(256, 4) kb_shade(BatchParams B) {
   __shared__ GroupDev sgd[BATCH_TABLE];
-  __shared__ ShadeSmem<256> sm;
+  __shared__ ShadeSmem<256, NRM, DENSE> sm;
   for (int i = threadIdx.x; i < B.ngroups; i += blockDim.x) sgd[i] = B.groups_draw[i];
   // the counters are final here; a copy a view took 3.5 us each of the copy
   // engine, which the read-backs need (nine views: 391 -> 354 us a pass)
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(256, 4) kb_shade(BatchParams B) {
       B.host_ctrs[i] = (V.kind == VIEW_DEPTH ? V.sp.ctr : V.dp.ctr)[i % CTR_N];
     }
   __syncthreads();
-  batch_shade<256, NRM>(B, sgd, sm);
+  batch_shade<256, NRM, DENSE>(B, sgd, sm);
 }
 
 }  // namespace axr

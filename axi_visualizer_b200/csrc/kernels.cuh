@@ -1806,9 +1806,14 @@ struct WinnerState {
   int y0;
 };
 // What its pixels need of the winner itself
-struct WinnerConst {
+struct WinnerBase {
   float fmip;
   int mip, g;
+};
+template <bool NRM>
+struct WinnerConst : WinnerBase {};
+template <>
+struct WinnerConst<true> : WinnerBase {
   V3 tan, bit;   // F_NORMAL: the triangle's tangent frame
 };
 
@@ -1834,30 +1839,36 @@ __device__ __forceinline__ void normal_frame(const Attr<false> a[3], const V3 p[
 // by 1 / rows, for the half walked upwards with the vertices exchanged.  Thread
 // 0 also takes the mip level, the group and (NRM, F_NORMAL groups) the tangent
 // frame.  NRM = false: draws without normal-mapped groups, whose shade then
-// carries none of that code.
-template <bool NRM>
+// carries none of that code.  PAIR: two threads set up the (winner, row) pair of
+// row cy instead, each all attributes along one edge, and make the additions up
+// to that row themselves.
+template <bool NRM, bool PAIR>
 __device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev *sg, uint32_t ord, int cy, int j,
-                                             WinnerState &w, WinnerConst &wc) {
-  const int role = j >> 1, k = j & 1;
+                                             WinnerState &w, RowState &rs, WinnerConst<NRM> &wc) {
+  const int k = j & 1;
+  int role = j >> 1;
   const uint32_t o = ord - 1;
   const bool tiled = (o >> 31) != 0, up = (o & 1) != 0;
   const uint32_t gtri = (o >> 1) & 0x3fffffffu;
   const int g = find_group(sg, P.ngroups, gtri);
   const GroupDev &G = sg[g];
   const int tri = (int)(gtri - G.tri_base);
-  V3 a[3];                       // the thread's attribute, in vertex order below
-  {
+  // a role's attribute of vertices p0, p1, p2
+  auto load = [&](V3 a[3], int role, int p0, int p1, int p2) {
     const float *src = role == 0 ? G.uv : role == 1 ? G.li : role == 2 ? G.vn : G.xyz;
-    const int n = role == 0 ? 2 : 3;
+    const int n = role == 0 ? 2 : 3, p[3] = {p0, p1, p2};
     src += (size_t)tri * 3 * n;
 #pragma unroll
-    for (int i = 0; i < 3; i++) a[i] = V3{__ldg(src + i * n), __ldg(src + i * n + 1), role == 0 ? 0.f : __ldg(src + i * n + 2)};
-  }
+    for (int i = 0; i < 3; i++)
+      a[i] = V3{__ldg(src + p[i] * n), __ldg(src + p[i] * n + 1), role == 0 ? 0.f : __ldg(src + p[i] * n + 2)};
+  };
+  V3 a[3];                       // the thread's attribute, in vertex order below
+  load(a, role, 0, 1, 2);
   float x[3], y[3], z[3];
   project_persp(G, tri, P.view, x, y, z);
-  int ix[3] = {0, 0, 0}, iy[3] = {0, 0, 0}, v0[3] = {0, 3, 6};   // v0: the vertices' offsets
+  int ix[3] = {0, 0, 0}, iy[3] = {0, 0, 0}, v0[3] = {0, 1, 2};   // v0: the vertices
   if (!tiled) {
-    // direct path: integer vertices (Templates.py:230-231)
+    // untiled path: integer vertices (Templates.py:230-231)
 #pragma unroll
     for (int i = 0; i < 3; i++) { ix[i] = f2i(x[i]); iy[i] = f2i(y[i]); }
   }
@@ -1869,11 +1880,9 @@ __device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev
   SW(0, 1)
 #undef SW
 #pragma unroll
-  for (int i = 0; i < 3; i++) {
-    a[i] = mul3(a[i], z[i]);
+  for (int i = 0; i < 3; i++)
     if (!tiled) x[i] = (float)ix[i];
-  }
-  // heights and x differences: of the integers on the direct path
+  // heights and x differences: of the integers on the untiled path
   float h21, h32, h31, x21, x32, x31;
   if (tiled) {
     h21 = y[1] - y[0]; h32 = y[2] - y[1]; h31 = y[2] - y[0];
@@ -1884,7 +1893,6 @@ __device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev
   }
   const float yd = h21 / h31;
   const float x4 = x[0] + yd * x31, z4 = z[0] + yd * (z[2] - z[0]);
-  const V3 a4 = add3(a[0], smul3(yd, sub3(a[2], a[0])));
   const bool mip = (G.flags & F_MIP) != 0, normal = NRM && (G.flags & F_NORMAL) != 0;
   if (j == 0) {
     wc.g = g;
@@ -1892,49 +1900,67 @@ __device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev
     wc.mip = 0;
     Attr<false> uv[3];
 #pragma unroll
-    for (int i = 0; i < 3; i++) uv[i].uv = V2{a[i].x, a[i].y};
-    if (normal) {
-      const float *xyz = G.xyz + (size_t)tri * 9;
-      V3 p[3] = {mul3(ld3(xyz + v0[0]), z[0]), mul3(ld3(xyz + v0[1]), z[1]), mul3(ld3(xyz + v0[2]), z[2])};
-      normal_frame(uv, p, z, wc.tan, wc.bit);
-    }
+    for (int i = 0; i < 3; i++) uv[i].uv = V2{a[i].x * z[i], a[i].y * z[i]};
+    if constexpr (NRM)
+      if (normal) {
+        const float *xyz = G.xyz + (size_t)tri * 9;
+        V3 p[3] = {mul3(ld3(xyz + 3 * v0[0]), z[0]), mul3(ld3(xyz + 3 * v0[1]), z[1]), mul3(ld3(xyz + 3 * v0[2]), z[2])};
+        normal_frame(uv, p, z, wc.tan, wc.bit);
+      }
     if (mip) {
       MipSel ms = mip_setup<false>(uv, z, !tiled, ix, iy, x, y, G.tex_size, G.mip_bias);
       wc.fmip = ms.fmip;
       wc.mip = ms.mip;
     }
   }
-  if ((mip || normal) && (role == 0 || role == 3)) {   // the round trip of uv and position (mip_setup)
-#pragma unroll
-    for (int i = 0; i < 3; i++) a[i] = mul3(div3(a[i], z[i]), z[i]);
-  }
   // the half's first vertex, its slopes to the middle and to the split vertex
   const float d = 1.0f / (up ? h32 : h21);
   const float xs = up ? x[2] : x[0], ys = up ? y[2] : y[0], zs = up ? z[2] : z[0];
   const float s1 = (up ? x32 : x21) * d, s2 = (up ? x[2] - x4 : x4 - x[0]) * d;
   const float sz = (k ? (up ? z[2] - z4 : z4 - z[0]) : (up ? z[2] - z[1] : z[1] - z[0])) * d, s = k ? s2 : s1;
-  const V3 from = up ? a[2] : a[0];
-  V3 sa = sub3(k ? a4 : a[1], from);
-  sa = mul3(up ? neg3(sa) : sa, d);
   const float yMin = (float)(cy / TILE) * 16.f;
   const int cy0 = tiled ? f2i(clampf_(ys, yMin, yMin + 15.f)) : (up ? iy[2] : iy[0]);
   const float dy = (float)cy0 - ys;          // tiled path: restarted at the tile's first row
   const int e = (s1 < s2) ? 1 - k : k;       // the larger slope is the first chain's
-  float *st = reinterpret_cast<float *>(&w.start[e]), *sp = reinterpret_cast<float *>(&w.step[e]);
-  const V3 c = tiled ? add3(from, smul3(dy, sa)) : from;
-  if (up) sa = neg3(sa);
+  const int rows = iabs_(cy - cy0);
+  float *st = reinterpret_cast<float *>(PAIR ? &rs.e[e] : &w.start[e]), *sp = reinterpret_cast<float *>(&w.step[e]);
   if (role == 0) {
-    st[0] = tiled ? xs + dy * s : xs;
-    st[1] = tiled ? zs + dy * sz : zs;
-    sp[0] = up ? -s : s;
-    sp[1] = up ? -sz : sz;
-    if (k == 0) w.y0 = cy0;
-    st[2] = c.x; st[3] = c.y;
-    sp[2] = sa.x; sp[3] = sa.y;
-  } else {
-    st += 1 + 3 * role; sp += 1 + 3 * role;
-    st[0] = c.x; st[1] = c.y; st[2] = c.z;
-    sp[0] = sa.x; sp[1] = sa.y; sp[2] = sa.z;
+    float cx = tiled ? xs + dy * s : xs, cz = tiled ? zs + dy * sz : zs;
+    const float sx = up ? -s : s, sw = up ? -sz : sz;
+    if (PAIR) {
+      for (int r = rows; r > 0; r--) { cx += sx; cz += sw; }
+    } else {
+      sp[0] = sx;
+      sp[1] = sw;
+      if (k == 0) w.y0 = cy0;
+    }
+    st[0] = cx;
+    st[1] = cz;
+  }
+#pragma unroll 1
+  while (true) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      a[i] = mul3(a[i], z[i]);
+      if ((mip || normal) && (role == 0 || role == 3))   // the round trip of uv and position (mip_setup)
+        a[i] = mul3(div3(a[i], z[i]), z[i]);
+    }
+    const V3 from = up ? a[2] : a[0], a4 = add3(a[0], smul3(yd, sub3(a[2], a[0])));
+    V3 sa = sub3(k ? a4 : a[1], from);
+    sa = mul3(up ? neg3(sa) : sa, d);
+    V3 c = tiled ? add3(from, smul3(dy, sa)) : from;
+    if (up) sa = neg3(sa);
+    const int at = role == 0 ? 2 : 1 + 3 * role;
+    if (PAIR) {
+      for (int r = rows; r > 0; r--) c = add3(c, sa);
+    } else {
+      sp[at] = sa.x; sp[at + 1] = sa.y;
+      if (role) sp[at + 2] = sa.z;
+    }
+    st[at] = c.x; st[at + 1] = c.y;
+    if (role) st[at + 2] = c.z;
+    if (!PAIR || ++role == 4) break;
+    load(a, role, v0[0], v0[1], v0[2]);
   }
 }
 
@@ -2043,7 +2069,7 @@ __device__ __forceinline__ V3 bilerp_nm(const Taps &q, const uchar4 *__restrict_
 // cascade (sample_shadow5), 1 without one.  Kept out of line so that the
 // other materials keep their registers.
 __device__ __forceinline__ void shade_normal(const DrawParams &P, const GroupDev &G, size_t pix, float t, float tz,
-                                          V2 uvi, const RowState &st, const WinnerConst &wc, MipSel ms) {
+                                          V2 uvi, const RowState &st, const WinnerConst<true> &wc, MipSel ms) {
   const Attr<true> &c1 = st.e[0].c, &c2 = st.e[1].c;
   const bool mip = (G.flags & F_MIP) != 0;
   float omt = 1 - t;
@@ -2123,7 +2149,7 @@ __device__ __forceinline__ void shade_normal(const DrawParams &P, const GroupDev
 // Shades pixel ax of row cy from its winner's row state.
 template <bool NRM = true>
 __device__ __forceinline__ void shade_from_row(const DrawParams &P, const GroupDev *sg, int ax, int cy,
-                                               const RowState &st, const WinnerConst &wc) {
+                                               const RowState &st, const WinnerConst<NRM> &wc) {
   const GroupDev &G = sg[wc.g];
   const bool mip = (G.flags & F_MIP) != 0;
   MipSel ms;
@@ -2142,10 +2168,11 @@ __device__ __forceinline__ void shade_from_row(const DrawParams &P, const GroupD
     shade_multi(P, &G, (size_t)P.view.w * cy + ax, t, tz, uvi, st);
     return;
   }
-  if (NRM && (G.flags & F_NORMAL)) {
-    shade_normal(P, G, (size_t)P.view.w * cy + ax, t, tz, uvi, st, wc, ms);
-    return;
-  }
+  if constexpr (NRM)
+    if (G.flags & F_NORMAL) {
+      shade_normal(P, G, (size_t)P.view.w * cy + ax, t, tz, uvi, st, wc, ms);
+      return;
+    }
   float outR, outG, outB;
   if (mip) {
     // av_draw_normmap_mip.c:73-123
@@ -2183,14 +2210,17 @@ __device__ __forceinline__ void shade_from_row(const DrawParams &P, const GroupD
 
 // Shared memory of shade_tile for a block of NT threads (16 x NT/16 pixels).
 constexpr int WINNERS = 32;        // winners set up at a time
-template <int NT>
+// DENSE: tiles with many winners of a row or two are set up by pair.
+template <int NT, bool NRM, bool DENSE>
 struct ShadeSmem {
+  // entries (winners, or pairs) shaded at a time: all, or with tangent frames what 48 KB hold
+  static constexpr int AT_ONCE = !NRM || NT <= 128 ? NT : DENSE ? 96 : WINNERS;
   uint32_t hkey[NT];               // open-addressing table of the tile's winners (order keys)
   uint16_t hent[NT];               // its entry numbers
   uint32_t ekey[NT];               // entry -> order key
   int nent, npair;
   uint16_t pair[NT];               // (winner, row) pairs: table slot << 4 | row
-  WinnerConst wc[WINNERS];
+  WinnerConst<NRM> wc[AT_ONCE];
   WinnerState ws[WINNERS];
   RowState rs[NT];                 // their edge chains, indexed alike
 };
@@ -2211,8 +2241,18 @@ struct ShadeSmem {
 // the barriers between the steps (6.9 of 14 cycles an instruction) with four
 // blocks of 64 registers an SM.  8-row tiles (half the threads a block) take 12%
 // longer; two or three blocks an SM 3-10%.
-template <int NT, bool NRM = true>
-__device__ __forceinline__ void shade_tile(const DrawParams &P, const GroupDev *sg, int x0, int y0, ShadeSmem<NT> &sm) {
+//
+// Every pixel shades in one pass after the last winners' set-up: with a pass after
+// each 32 winners a warp of a tile with many of them shaded up to eight times.  And
+// where winners are nearly as many as pairs (fine meshes in small views), two
+// threads a pair take fewer rounds than eight a winner (DENSE, by_pair).  k_shade with
+// every pair set up by itself, by winner with a pass after each 32, now: 1.04M
+// triangles at 64x48 31, 74, 33 us; at 320x192 from above 37, 81, 35; 2.9M at 640x480
+// from above 75, 142, 75; 300,000 at 720p from above 109, 137, 122; from the side
+// 99, 80, 78.
+template <int NT, bool NRM, bool DENSE>
+__device__ __forceinline__ void shade_tile(const DrawParams &P, const GroupDev *sg, int x0, int y0,
+                                           ShadeSmem<NT, NRM, DENSE> &sm) {
   const int tid = threadIdx.x, lane = tid & 31;
   const int ax = x0 + (tid & 15), cy = y0 + (tid >> 4);
   const bool in = ax < P.view.w && cy < P.view.h;
@@ -2246,35 +2286,54 @@ __device__ __forceinline__ void shade_tile(const DrawParams &P, const GroupDev *
   if (leads) sm.pair[pair] = (uint16_t)(slot << 4 | tid >> 4);
   __syncthreads();
   const int nw = sm.nent, npairs = sm.npair;
-  for (int base = 0; base < nw; base += WINNERS) {
-    const int m = min(WINNERS, nw - base);
-    for (int j = tid; j < 8 * m; j += NT)
-      winner_setup<NRM>(P, sg, sm.ekey[base + (j >> 3)], y0, j & 7, sm.ws[j >> 3], sm.wc[j >> 3]);
-    __syncthreads();
-    for (int j = tid; j < 2 * npairs; j += NT) {
-      const int info = sm.pair[j >> 1], w = (int)sm.hent[info >> 4] - base;
-      if ((unsigned)w < (unsigned)m) replay_edge(sm.ws[w], j & 1, y0 + (info & 15), sm.rs[j >> 1].e[j & 1]);
+  sm.hkey[tid] = ord ? pair + 1u : 0u;   // (the keys are not read again) kept there, not in a register
+  constexpr int AT_ONCE = ShadeSmem<NT, NRM, DENSE>::AT_ONCE;
+  constexpr bool ALL = AT_ONCE == NT;    // one pass of the outer loop
+  // a round of pairs costs about twice one of winners
+  const bool by_pair = DENSE && (nw + WINNERS - 1) / WINNERS > 2 * ((2 * npairs + NT - 1) / NT);
+  const int total = by_pair ? npairs : nw;
+  for (int c0 = 0; c0 < (ALL ? 1 : total); c0 += AT_ONCE) {
+    const int n = ALL ? total : min(AT_ONCE, total - c0);
+    if (by_pair) {
+      for (int j = tid; j < 2 * n; j += NT) {
+        const int i = c0 + (j >> 1), info = sm.pair[i];
+        winner_setup<NRM, true>(P, sg, sm.ekey[sm.hent[info >> 4]], y0 + (info & 15), j & 1, sm.ws[0], sm.rs[i], sm.wc[j >> 1]);
+      }
+      __syncthreads();
+    } else {
+      for (int base = c0; base < c0 + n; base += WINNERS) {
+        const int m = min(WINNERS, c0 + n - base);
+        for (int j = tid; j < 8 * m; j += NT)
+          winner_setup<NRM, false>(P, sg, sm.ekey[base + (j >> 3)], y0, j & 7, sm.ws[j >> 3], sm.rs[0], sm.wc[base - c0 + (j >> 3)]);
+        __syncthreads();
+        for (int j = tid; j < 2 * npairs; j += NT) {
+          const int info = sm.pair[j >> 1], w = (int)sm.hent[info >> 4] - base;
+          if ((unsigned)w < (unsigned)m) replay_edge(sm.ws[w], j & 1, y0 + (info & 15), sm.rs[j >> 1].e[j & 1]);
+        }
+        __syncthreads();
+      }
     }
-    __syncthreads();
-    if (ord != 0) {
-      const int w = (int)sm.hent[sm.pair[pair] >> 4] - base;
-      if ((unsigned)w < (unsigned)m) shade_from_row<NRM>(P, sg, ax, cy, sm.rs[pair], sm.wc[w]);
+    const int mine = (int)sm.hkey[tid] - 1;
+    if (mine >= 0) {
+      const int w = (by_pair ? mine : (int)sm.hent[sm.pair[mine] >> 4]) - c0;
+      if (ALL || (unsigned)w < (unsigned)n)
+        shade_from_row<NRM>(P, sg, x0 + (tid & 15), y0 + (tid >> 4), sm.rs[mine], sm.wc[w]);
     }
-    __syncthreads();                     // the next winners (or the next tile) reuse the shared memory
+    __syncthreads();                     // the next entries (or the next tile) reuse the shared memory
   }
 }
 
 // one 256-thread block per 16x16 tile
 // NRM: the draw has normal-mapped groups
-template <bool NRM>
+template <bool NRM, bool DENSE>
 __global__ void __launch_bounds__(256, 4) k_shade(DrawParams P) {   // 64 registers: 4 blocks per SM
   __shared__ GroupDev sg[64];
-  __shared__ ShadeSmem<256> sm;
+  __shared__ ShadeSmem<256, NRM, DENSE> sm;
   for (int i = threadIdx.x; i < P.ngroups; i += blockDim.x) sg[i] = P.groups[i];
   if (P.host_ctr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < CTR_N)
     P.host_ctr[threadIdx.x] = P.ctr[threadIdx.x];     // final: every kernel that counts has finished
   __syncthreads();
-  shade_tile<256, NRM>(P, sg, blockIdx.x * TILE, blockIdx.y * TILE, sm);
+  shade_tile<256, NRM, DENSE>(P, sg, blockIdx.x * TILE, blockIdx.y * TILE, sm);
 }
 
 __global__ void k_ids(const uint64_t *__restrict__ keys, int n, int32_t *tri_id, uint8_t *cov) {
