@@ -112,9 +112,13 @@ struct Shadow {
 };
 
 constexpr int MAX_GROUPS = 64;
-// from this many triangles the alpha-tested rasterizers run on their own stream
-// (2,512 triangles at 320x192: 99 us a frame among others without, 107 with
-// it, alone 190 and 171; 301,000 at 720p: 452 alone without, 385 with it)
+// From this many triangles the alpha-tested rasterizers run on their own stream.
+// Without it, with it, in us a frame among others (alone), scenes with 10% of
+// alpha-tested triangles: 320x192 2,418 triangles 103 (186) and 108 (170), 12,002
+// 100 (197), 104 (180); 1280x720 2,418 107 (268), 107 (235), 5,028 116 (285), 111
+// (250), 12,002 136 (304), 127 (260); 1920x1080 5,028 199 (369), 195 (325).  So one
+// stream pays only among other small views, where the host's calls bound the
+// frame; the line is by triangles, as the launches do not know what is visible.
 constexpr int SIDE_STREAM_TRIS = 8192;
 // Rows per work item where no tuning is set: 20 for casters, and for the small
 // triangles of large scenes, 12 (MIN_CHUNK) for those of others.  Setting an
@@ -122,7 +126,11 @@ constexpr int SIDE_STREAM_TRIS = 8192;
 // instructions; shorter ones spread a small view's work over more warps.  With 12
 // throughout the 4K / 2.9M-triangle frame took 2149 us, casters at 20 2043, both
 // 2019; 1080p / 1.04M 813, 798, 790; 720p / 300k 292, 287, 285, but alone 382,
-// 382, 397, and the normal-mapped 1296x713 view 157, 157, 165.
+// 382, 397, and the normal-mapped 1296x713 view 157, 157, 165.  The view at 12 and
+// 20 (casters at 20), among others (alone): 720p / 450k 283 (385) and 284 (394), 600k
+// 323 (420), 324 (436), 800k 377 (486), 377 (494); 1080p / 600k 588 (661), 587 (671),
+// 1.6M 981 (1104), 971 (1112); 4K / 1M 1605 (1703), 1597 (1694).  The line matters
+// little between 300,000 and 1M triangles.
 constexpr int LONG_ITEM = 20, LONG_ITEM_TRIS = 700000;
 // From 1.5 drawn triangles a pixel the shade has the set-up by pair of row and
 // winner (its tiles may then hold up to 256 winners of a row each).  That code

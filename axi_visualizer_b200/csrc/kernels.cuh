@@ -89,7 +89,7 @@ __device__ __forceinline__ void span_clip(int ax0, float bound, int w, int &lo, 
 // rows, so that large "small" triangles spread over several lanes; a lane
 // replays the row accumulation up to its chunk, which keeps every
 // interpolant bit-identical to the serial walk.
-constexpr int MIN_CHUNK = 12;   // default of DrawParams::min_chunk
+constexpr int MIN_CHUNK = 12;   // DrawParams::min_chunk of smaller scenes and of batches where no tuning is set
 constexpr int CHUNK_BITS = 3;   // work item = list position << CHUNK_BITS | chunk
 constexpr int MAX_CHUNKS = 1 << CHUNK_BITS;
 __device__ __forceinline__ int small_rows(int y1, int y3) { return y3 - y1 + 2; }
@@ -810,7 +810,8 @@ __device__ __forceinline__ void block_reserve(const uint32_t (&v)[K], const int 
 }
 
 // Writes the row-chunk work items of a block's triangles (or casters),
-// sorted by their row count, longest first, into one region per kind and
+// sorted by their row count, longest first (15 rows and more share a bucket and
+// are not ordered among themselves), into one region per kind and
 // block (opaque items from the front of `items`, alpha-tested ones from the
 // back).  A warp of the raster claims 32 consecutive items, so sorted items
 // give it rows of about the same count, and fewer lanes idle while the
@@ -2066,8 +2067,9 @@ __device__ __forceinline__ V3 bilerp_nm(const Taps &q, const uchar4 *__restrict_
 // The normal-mapped fragment cores: av_draw_normmap.c:47-149 (its alpha
 // variant after the visibility pass's alpha test) and, with F_MIP,
 // av_draw_normmap_mip.c:73-160.  The light comes from the draw's first
-// cascade (sample_shadow5), 1 without one.  Kept out of line so that the
-// other materials keep their registers.
+// cascade (sample_shadow5), 1 without one.  Inlined, as its arguments went
+// through local memory otherwise; draws without such a material launch a shade
+// without this code.
 __device__ __forceinline__ void shade_normal(const DrawParams &P, const GroupDev &G, size_t pix, float t, float tz,
                                           V2 uvi, const RowState &st, const WinnerConst<true> &wc, MipSel ms) {
   const Attr<true> &c1 = st.e[0].c, &c2 = st.e[1].c;
@@ -2374,10 +2376,10 @@ struct ShadowParams {
   int sort;            // 1: each tile's units front (nearest the light) first
 };
 
-// Rows per work item of a caster (at least).  Alpha-tested casters take
-// half: their fragments cost more (the mask), so they balance better over
-// shorter items (on the 1080p scene's cascades 102 -> 86 us at 6 rows
-// against 12, while the opaque casters are fastest at 12).
+// Rows per work item of a caster (at least).  Alpha-tested casters take half:
+// their fragments cost more (the mask), so they balance better over shorter
+// items (an earlier build took 86 us for the 1080p scene's cascades with 6 rows
+// and 102 with 12; it is 10 and 20 rows now, see LONG_ITEM).
 __device__ __forceinline__ int shadow_min_chunk(const ShadowParams &S, bool alpha) {
   return alpha ? max(1, S.min_chunk >> 1) : S.min_chunk;
 }
@@ -2890,9 +2892,9 @@ __device__ __forceinline__ void shadow_warp_loop(const ShadowParams &S, const Gr
   }
 }
 
-// Blocks per SM: the opaque casters fit 9 in 56 registers and the
-// alpha-tested ones 7 in 72, neither spilling (204 -> 199 and 84 -> 80 us
-// per cascade against 8 and 6 blocks).
+// Blocks per SM: the opaque casters fit 9 in 56 registers without spills, the
+// alpha-tested ones 7 in 72 with 20 bytes of them.  With an earlier build of both
+// 204 -> 199 and 84 -> 80 us per cascade against 8 and 6 blocks.
 template <bool ALPHA>
 __global__ void __launch_bounds__(128, ALPHA ? 7 : 9) k_shadow_raster(ShadowParams S) {
   __shared__ GroupDev sg[64];
