@@ -1881,8 +1881,10 @@ __device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev
   SW(0, 1)
 #undef SW
 #pragma unroll
-  for (int i = 0; i < 3; i++)
+  for (int i = 0; i < 3; i++) {
+    a[i] = mul3(a[i], z[i]);
     if (!tiled) x[i] = (float)ix[i];
+  }
   // heights and x differences: of the integers on the untiled path
   float h21, h32, h31, x21, x32, x31;
   if (tiled) {
@@ -1901,7 +1903,7 @@ __device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev
     wc.mip = 0;
     Attr<false> uv[3];
 #pragma unroll
-    for (int i = 0; i < 3; i++) uv[i].uv = V2{a[i].x * z[i], a[i].y * z[i]};
+    for (int i = 0; i < 3; i++) uv[i].uv = V2{a[i].x, a[i].y};
     if constexpr (NRM)
       if (normal) {
         const float *xyz = G.xyz + (size_t)tri * 9;
@@ -1940,11 +1942,9 @@ __device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev
   }
 #pragma unroll 1
   while (true) {
+    if ((mip || normal) && (role == 0 || role == 3)) {   // the round trip of uv and position (mip_setup)
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-      a[i] = mul3(a[i], z[i]);
-      if ((mip || normal) && (role == 0 || role == 3))   // the round trip of uv and position (mip_setup)
-        a[i] = mul3(div3(a[i], z[i]), z[i]);
+      for (int i = 0; i < 3; i++) a[i] = mul3(div3(a[i], z[i]), z[i]);
     }
     const V3 from = up ? a[2] : a[0], a4 = add3(a[0], smul3(yd, sub3(a[2], a[0])));
     V3 sa = sub3(k ? a4 : a[1], from);
@@ -1962,6 +1962,8 @@ __device__ __forceinline__ void winner_setup(const DrawParams &P, const GroupDev
     if (role) st[at + 2] = c.z;
     if (!PAIR || ++role == 4) break;
     load(a, role, v0[0], v0[1], v0[2]);
+#pragma unroll
+    for (int i = 0; i < 3; i++) a[i] = mul3(a[i], z[i]);
   }
 }
 
