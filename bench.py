@@ -44,24 +44,24 @@ FALLBACK_HBM_GBS = 6650.0
 # names the committed summary of that capture, reported in the JSON line.
 NCU_CAPTURE = "profiles/ncu_kernels_1080p_1m.md"
 NCU_TRAFFIC = {
-    "k_raster_small": 32811008,
-    "k_raster_small_alpha": 13467648,
-    "k_shadow_raster": (46954496 + 50692096) // 2,
-    "k_shadow_raster_alpha": (10293248 + 4461568) // 2,
-    "k_shade": 30253056,
-    "k_raster_tiled": 10337280,
-    "k_raster_tiled_alpha": 8160256,
-    "k_shadow_setup": (37618944 + 37617920) // 2,
-    "k_setup": 54932224,
+    "k_raster_small": 32813824,
+    "k_raster_small_alpha": 13466624,
+    "k_shadow_raster": (46949632 + 50689024) // 2,
+    "k_shadow_raster_alpha": (10291200 + 4465152) // 2,
+    "k_shade": 30319872,
+    "k_raster_tiled": 10353408,
+    "k_raster_tiled_alpha": 8158464,
+    "k_shadow_setup": (37617920 + 37619712) // 2,
+    "k_setup": 54958336,
 }
 NCU_ISSUED = {
-    "k_raster_small": 83089658,
-    "k_raster_small_alpha": 69438194,
-    "k_shadow_raster": 144353943 + 83025235,
-    "k_shadow_raster_alpha": 34789834 + 12203377,
-    "k_shade": 78040365,
-    "k_raster_tiled": 20877990,
-    "k_raster_tiled_alpha": 29736853,
+    "k_raster_small": 83122508,
+    "k_raster_small_alpha": 69508703,
+    "k_shadow_raster": 144633043 + 83271446,
+    "k_shadow_raster_alpha": 34890508 + 12303716,
+    "k_shade": 77281168,
+    "k_raster_tiled": 20897991,
+    "k_raster_tiled_alpha": 29877438,
     "k_shadow_setup": 14444480 + 14714699,
     "k_setup": 14435226,
 }
